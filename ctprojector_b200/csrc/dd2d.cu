@@ -37,6 +37,7 @@
 #include <type_traits>
 
 #include "ctp_common.cuh"
+#include "dd2d_gather.cuh"
 
 namespace ctp {
 
@@ -1289,576 +1290,6 @@ __global__ void __launch_bounds__(256, (fp_stream_min_blocks<FAN, NI>())) dd2d_f
     }
 }
 
-// ---------------------------------------------------------------------------
-// Parallel-beam normalised back projection, fast path.
-//
-// For a parallel beam the detector coordinate of a pixel centre,
-// jc = -((x cos + y sin)/du + off_u) + nu/2, is linear in (ix, iy) with steps
-// jx = -dx cos/du and jy = -dy sin/du, and the footprint of the pixel's
-// x-edges is [jc - |jx|/2, jc + |jx|/2] (of its y-edges, jc -+ |jy|/2).  The
-// reference's normalised box integral (DDBPParallelKernel,
-// distanceDriven2DBoxInt.cu:409-497) is then (F(e1) - F(e0)) / (e1 - e0) with
-// F the running integral of the detector row, and neighbouring pixels share
-// footprint edges: pixels ix and ix+1 meet at jc + jx/2.  So a thread that
-// owns 4 consecutive pixels along x evaluates F at 5 edges for the x-edge
-// term, and one that owns 4 consecutive pixels along y does the same for the
-// y-edge term.  Each thread holds one pixel run of each kind (x-layout and
-// y-layout accumulators) and the two are added through shared memory at the
-// end.
-//
-// A CTA owns a 32x32 tile of one slice.  Per chunk of 32 views: one thread per
-// view computes the view's constants in FP64 (tile-origin coordinate, steps,
-// blend weights, staged window); each warp then stages, for its views, the
-// window of cells the tile projects onto as a midpoint table of window-local
-// running sums (small, so FP32 keeps them accurate); then every thread adds
-// the views to its 8 pixels with table lookups only.  No atomics.
-constexpr int kPT = 32;        // tile edge
-constexpr int kPViews = 32;    // views per staged chunk
-constexpr int kPMaxWin = 255;  // staged cells per view (table holds win+1 entries)
-
-// Window tables of the fast back projectors, staged by one warp M at a time:
-// for each item, entries k = 0 .. win of (running sum of the window cells
-// before k + value/2, value) for the cells w0 .. w0 + win - 1 of the detector
-// row at `row` (cells off the detector, and the entry past the window, are
-// zero; ok = false stages zeros, valid = false writes nothing).  Lane l scans
-// the PER consecutive entries from l PER of every item: it issues all M PER
-// loads before it sums, so that the items' load latencies overlap, then the
-// warp scans the lane sums and the lane writes its entries.
-template <typename Tp>
-struct WinItem {
-    float2* T;
-    const Tp* row;
-    int w0;
-    bool ok, valid;
-};
-// Windows a warp stages together: on the parallel 16 x 512^2, 720-view batch
-// the back projection takes 1.97, 1.75 and 1.90 ms with 1, 2 and 4 (4 spills).
-constexpr int kStageBatch = 2;
-
-template <int PER, int M, typename Tp>
-__device__ __forceinline__ void stage_windows_per(const WinItem<Tp> (&it)[M], int win, int nu, int lane) {
-    const int k0 = lane * PER;
-    float v[M][PER];
-    float run[M], incl[M];
-#pragma unroll
-    for (int m = 0; m < M; ++m)
-#pragma unroll
-        for (int q = 0; q < PER; ++q) {
-            const int k = k0 + q, cell = it[m].w0 + k;
-            v[m][q] = (it[m].ok && k < win && cell >= 0 && cell < nu) ? ldf(it[m].row + cell) : 0.f;
-        }
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-        run[m] = 0.f;
-#pragma unroll
-        for (int q = 0; q < PER; ++q) run[m] += v[m][q];
-        incl[m] = run[m];
-    }
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1)
-#pragma unroll
-        for (int m = 0; m < M; ++m) {
-            const float t = __shfl_up_sync(0xffffffffu, incl[m], o);
-            if (lane >= o) incl[m] += t;
-        }
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-        if (!it[m].valid) continue;
-        float base = incl[m] - run[m];
-#pragma unroll
-        for (int q = 0; q < PER; ++q) {
-            const int k = k0 + q;
-            if (k <= win) it[m].T[k] = make_float2(fmaf(0.5f, v[m][q], base), v[m][q]);
-            base += v[m][q];
-        }
-    }
-}
-
-// The same for any window of up to 255 cells: PER = ceil((win + 1) / 32),
-// a compile-time count, so a lane issues exactly its loads.
-template <int M, typename Tp>
-__device__ __forceinline__ void stage_windows(const WinItem<Tp> (&it)[M], int win, int nu, int lane) {
-    switch ((win + 1 + 31) / 32) {
-        case 1: stage_windows_per<1>(it, win, nu, lane); break;
-        case 2: stage_windows_per<2>(it, win, nu, lane); break;
-        case 3: stage_windows_per<3>(it, win, nu, lane); break;
-        case 4: stage_windows_per<4>(it, win, nu, lane); break;
-        case 5: stage_windows_per<5>(it, win, nu, lane); break;
-        case 6: stage_windows_per<6>(it, win, nu, lane); break;
-        case 7: stage_windows_per<7>(it, win, nu, lane); break;
-        default: stage_windows_per<8>(it, win, nu, lane); break;
-    }
-}
-
-struct ParView {
-    float jb, jx, jy, sx;  // jb: window coordinate - 1/2 of the tile's first pixel centre
-    float sy, jc, hx, hy;  // sx, sy: signed normalisations (0 = term inactive); jc: absolute coordinate
-};
-
-inline size_t par_fast_smem(int win, int S) {
-    return (size_t)S * kPViews * (win + 1) * sizeof(float2) + kPViews * sizeof(ParView) + kPViews * sizeof(int) +
-           (size_t)S * kPT * (kPT + 1) * sizeof(float);
-}
-
-// S slices of the same geometry per CTA: the per-view constants, the edge
-// positions and each lookup's index and fraction are shared; only the table
-// reads and the sums repeat per slice.
-// Views are split over blockIdx.z in parts of vper (a multiple of kPViews)
-// when the tile grid alone leaves SMs idle or fills its last wave poorly
-// (bp_view_parts); part z writes its own partial volume at
-// img + z * part_elems (summed by bp_parts_sum_kernel).
-template <typename Tp, typename Tout, int S>
-__global__ void __launch_bounds__(256) dd2d_bp_par_fast_kernel(Tout* __restrict__ img, const Tp* __restrict__ prj,
-                                                               const float* __restrict__ deg, int nview, Grid g,
-                                                               Det d, int fbp, int accumulate, int win,
-                                                               int nslices, int vper, size_t part_elems) {
-    extern __shared__ float4 smem_f4[];
-    const int stride = win + 1;
-    float2* s_tab = reinterpret_cast<float2*>(smem_f4);                       // [S][kPViews][stride]
-    ParView* s_par = reinterpret_cast<ParView*>(s_tab + S * kPViews * stride);  // 16-byte aligned: 256 * S * stride bytes before
-    int* s_w0 = reinterpret_cast<int*>(s_par + kPViews);                      // window start, INT_MIN = not staged
-    float* s_acc = reinterpret_cast<float*>(s_w0 + kPViews);                  // [S][kPT][kPT + 1] merge buffer
-
-    const int tiles_x = (g.nx + kPT - 1) / kPT;
-    const int tx0 = (blockIdx.x % tiles_x) * kPT, ty0 = (blockIdx.x / tiles_x) * kPT;
-    const int s0 = blockIdx.y * S;  // first slice (b * nz + iz) of this CTA
-    const int ns = min(S, nslices - s0);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // x-layout: 4 pixels along x; a half warp spans 16 columns x 4 rows, so its
-    // table reads fall on distinct banks.  y-layout: 4 pixels along y, lane = column.
-    const int xl_row = warp * 4 + ((lane >> 2) & 3);
-    const int xl_col = ((lane >> 4) * 4 + (lane & 3)) * 4;
-    const int yl_col = lane, yl_row = warp * 4;
-
-    // detector row of each slice (truncation, :383); a slice off the detector stages zeros
-    const Tp* rows[S];
-    bool row_ok[S];
-    bool any_row = false;
-#pragma unroll
-    for (int s = 0; s < S; ++s) {
-        const int slice = s0 + min(s, ns - 1), iz = slice % g.nz, b = slice / g.nz;
-        const float zc = ((float)iz - g.nz / 2.f) * g.dz + g.cz + g.dz / 2;
-        const int iv = (int)(zc / d.dv + d.off_v + d.nv / 2.f - 0.5f);
-        row_ok[s] = s < ns && iv >= 0 && iv < d.nv;
-        rows[s] = prj + ((size_t)b * nview * d.nv + (row_ok[s] ? iv : 0)) * d.nu;
-        any_row |= row_ok[s];
-    }
-    float ax[S][4], ay[S][4];
-#pragma unroll
-    for (int s = 0; s < S; ++s)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) ax[s][k] = ay[s][k] = 0.f;
-    const size_t vstride = (size_t)d.nv * d.nu;
-    const size_t tstride = (size_t)kPViews * stride;  // per slice
-
-    img += blockIdx.z * part_elems;
-    const int vb = blockIdx.z * vper, ve = min(nview, vb + vper);
-    for (int v0 = vb; v0 < ve && any_row; v0 += kPViews) {
-        const int nvc = min(kPViews, ve - v0);
-        if (threadIdx.x < nvc) {
-            const int vi = threadIdx.x, view = v0 + vi;
-            double s, c;
-            sincos((double)deg[view], &s, &c);
-            const double du = d.du;
-            const double jx = -c * g.dx / du, jy = -s * g.dy / du;
-            const double xc0 = (tx0 + 0.5 - 0.5 * g.nx) * g.dx + g.cx;
-            const double yc0 = (ty0 + 0.5 - 0.5 * g.ny) * g.dy + g.cy;
-            const double j00 = -((xc0 * c + yc0 * s) / du + d.off_u) + 0.5 * d.nu;
-            const double ac = fabs(c), as = fabs(s);
-            const bool ya = ac > as - kDDMarginD, xa = ac < as + kDDMarginD;
-            const double r = (ac - as + kDDMarginD) / (2 * kDDMarginD);
-            const double wx = r < 0 ? 0.0 : (r > 1 ? 1.0 : r);
-            const double hx = 0.5 * g.dx * ac / du, hy = 0.5 * g.dy * as / du;
-            const double hm = fmax(ya ? hx : 0.0, xa ? hy : 0.0);
-            const double pw = fbp ? 1.0 : (ref_y_main(deg[view]) ? g.dy / ac : g.dx / as);  // Utils.cu:39-65
-            const double jmin = j00 + fmin(0.0, (kPT - 1) * jx) + fmin(0.0, (kPT - 1) * jy);
-            const double jmax = j00 + fmax(0.0, (kPT - 1) * jx) + fmax(0.0, (kPT - 1) * jy);
-            bool ok = isfinite(j00) && isfinite(hm);
-            int w0 = 0;
-            if (ok) {
-                // two spare cells on each side: every edge lookup lands in [1.5, win - 2.5]
-                w0 = (int)floor(jmin - hm) - 2;
-                ok = ((int)ceil(jmax + hm) + 2 - w0) <= win;
-            }
-            ParView P;
-            P.jb = (float)(j00 - w0 - 0.5);
-            P.jx = (float)jx;
-            P.jy = (float)jy;
-            P.sx = ya ? (float)(pw * wx / jx) : 0.f;
-            P.sy = xa ? (float)(pw * (1 - wx) / jy) : 0.f;
-            P.jc = (float)j00;
-            P.hx = (float)hx;
-            P.hy = (float)hy;
-            s_par[vi] = P;
-            s_w0[vi] = ok ? w0 : INT_MIN;
-        }
-        __syncthreads();
-        // stage (running sum + value/2, value) for window cells w0 .. w0+win-1; entry win = (total, 0)
-        for (int sv0 = warp; sv0 < S * nvc; sv0 += 8 * kStageBatch) {
-            WinItem<Tp> it[kStageBatch];
-#pragma unroll
-            for (int m = 0; m < kStageBatch; ++m) {
-                const int sv = sv0 + 8 * m;
-                const int s = sv / nvc, vi = sv - s * nvc;
-                const Tp* srow = rows[0];
-                bool rok = row_ok[0];
-#pragma unroll
-                for (int q = 1; q < S; ++q)
-                    if (s == q) {
-                        srow = rows[q];
-                        rok = row_ok[q];
-                    }
-                it[m].valid = sv < S * nvc;
-                it[m].w0 = s_w0[vi];
-                it[m].ok = it[m].valid && it[m].w0 != INT_MIN && rok;
-                it[m].T = s_tab + s * tstride + vi * stride;
-                it[m].row = srow + (size_t)(v0 + vi) * vstride;
-            }
-            stage_windows(it, win, d.nu, lane);
-        }
-        __syncthreads();
-        for (int vi = 0; vi < nvc; ++vi) {
-            const ParView P = s_par[vi];
-            const float2* T = s_tab + vi * stride;
-            if (s_w0[vi] != INT_MIN) {
-                if (P.sx != 0.f) {
-                    const float e0 = fmaf((float)xl_col - 0.5f, P.jx, fmaf((float)xl_row, P.jy, P.jb));
-                    float f[S][5];
-#pragma unroll
-                    for (int k = 0; k < 5; ++k) {
-                        const float xs = fmaf((float)k, P.jx, e0);
-                        const float tt = xs + kRoundMagic;
-                        const int i = __float_as_int(tt) - kRoundMagicBits;
-                        const float fr = xs - (tt - kRoundMagic);
-#pragma unroll
-                        for (int s = 0; s < S; ++s) {
-                            const float2 e = T[s * tstride + i];
-                            f[s][k] = fmaf(e.y, fr, e.x);
-                        }
-                    }
-#pragma unroll
-                    for (int s = 0; s < S; ++s)
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) ax[s][k] = fmaf(f[s][k + 1] - f[s][k], P.sx, ax[s][k]);
-                }
-                if (P.sy != 0.f) {
-                    const float e0 = fmaf((float)yl_row - 0.5f, P.jy, fmaf((float)yl_col, P.jx, P.jb));
-                    float f[S][5];
-#pragma unroll
-                    for (int k = 0; k < 5; ++k) {
-                        const float xs = fmaf((float)k, P.jy, e0);
-                        const float tt = xs + kRoundMagic;
-                        const int i = __float_as_int(tt) - kRoundMagicBits;
-                        const float fr = xs - (tt - kRoundMagic);
-#pragma unroll
-                        for (int s = 0; s < S; ++s) {
-                            const float2 e = T[s * tstride + i];
-                            f[s][k] = fmaf(e.y, fr, e.x);
-                        }
-                    }
-#pragma unroll
-                    for (int s = 0; s < S; ++s)
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) ay[s][k] = fmaf(f[s][k + 1] - f[s][k], P.sy, ay[s][k]);
-                }
-            } else {
-                // window larger than the staging buffer: integrate the rows in global memory
-#pragma unroll
-                for (int s = 0; s < S; ++s) {
-                    if (!row_ok[s]) continue;
-                    const Tp* grow = rows[s] + (size_t)(v0 + vi) * vstride;
-                    if (P.sx != 0.f) {
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            float jc = P.jc + (float)(xl_col + k) * P.jx + (float)xl_row * P.jy;
-                            ax[s][k] += box_line(grow, 1, jc - P.hx, jc + P.hx, d.nu) * fabsf(P.sx);
-                        }
-                    }
-                    if (P.sy != 0.f) {
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            float jc = P.jc + (float)yl_col * P.jx + (float)(yl_row + k) * P.jy;
-                            ay[s][k] += box_line(grow, 1, jc - P.hy, jc + P.hy, d.nu) * fabsf(P.sy);
-                        }
-                    }
-                }
-            }
-        }
-        __syncthreads();
-    }
-    // add the x-layout sums to the y-layout ones and store rows coalesced
-#pragma unroll
-    for (int s = 0; s < S; ++s)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) s_acc[(s * kPT + xl_row) * (kPT + 1) + xl_col + k] = ax[s][k];
-    __syncthreads();
-    const int ix = tx0 + yl_col;
-#pragma unroll
-    for (int s = 0; s < S; ++s) {
-        if (s >= ns) continue;
-        const int slice = s0 + s, iz = slice % g.nz, b = slice / g.nz;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            int iy = ty0 + yl_row + k;
-            if (ix < g.nx && iy < g.ny) {
-                Tout* o = img + (((size_t)b * g.nz + iz) * g.ny + iy) * g.nx + ix;
-                float a = ay[s][k] + s_acc[(s * kPT + yl_row + k) * (kPT + 1) + yl_col];
-                if (accumulate) a += rdf(o);
-                stf(o, a);
-            }
-        }
-    }
-}
-
-// Fan-beam normalised back projection (and FBP weighting), fast path.
-// DDBPFanKernel (distanceDriven2DBoxInt.cu:319-396): per pixel and view, the
-// pixel's x-edges at its centre row (or y-edges at its centre column, by the
-// reference's intrinsic axis switch) are mapped to the detector with
-// atan(rx / (ry + dso)) (distanceDriven2DUtils.cu:96-101) and the pre-weighted
-// row is integrated between them and normalised by the mapped width.  Pixels
-// next to each other along the switched axis share an edge point, so a thread
-// owning 4 consecutive pixels along that axis maps 5 edge points, not 8: the
-// x-layout of the parallel path for x-edge views, the y-layout for y-edge
-// views, merged through shared memory at the end.  Same tiling and window
-// tables as the parallel fast path; src is the pre-weighted sinogram (or the
-// plain one in FBP mode).
-struct FanView {
-    float c, s;
-    int w0;  // window start, INT_MIN = not staged
-    int ym;  // x-edges at the centre row (1) or y-edges at the centre column (0)
-};
-
-inline size_t fan_fast_smem(int win, int S) {
-    return (size_t)S * kPViews * (win + 1) * sizeof(float2) + kPViews * sizeof(FanView) +
-           (size_t)S * kPT * (kPT + 1) * sizeof(float);
-}
-
-// S slices of the same geometry per CTA: the atan mappings of the edge points,
-// the footprint widths, the FBP weights and each lookup's index and fraction
-// are shared; only the table reads and sums repeat per slice.
-template <typename Tp, typename Tout, int S>
-__global__ void __launch_bounds__(256) dd2d_bp_fan_fast_kernel(Tout* __restrict__ img, const Tp* __restrict__ src,
-                                                               const float* __restrict__ deg, int nview, Grid g,
-                                                               Det d, float dso, int fbp, int accumulate, int win,
-                                                               int nslices, int vper, size_t part_elems) {
-    extern __shared__ float4 smem_f4[];
-    const int stride = win + 1;
-    float2* s_tab = reinterpret_cast<float2*>(smem_f4);                        // [S][kPViews][stride]
-    FanView* s_view = reinterpret_cast<FanView*>(s_tab + S * kPViews * stride);
-    float* s_acc = reinterpret_cast<float*>(s_view + kPViews);                 // [S][kPT][kPT + 1] merge buffer
-
-    const int tiles_x = (g.nx + kPT - 1) / kPT;
-    const int tx0 = (blockIdx.x % tiles_x) * kPT, ty0 = (blockIdx.x / tiles_x) * kPT;
-    const int s0 = blockIdx.y * S;
-    const int ns = min(S, nslices - s0);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int xl_row = warp * 4 + ((lane >> 2) & 3);
-    const int xl_col = ((lane >> 4) * 4 + (lane & 3)) * 4;
-    const int yl_col = lane, yl_row = warp * 4;
-
-    const Tp* rows[S];
-    bool row_ok[S];
-    bool any_row = false;
-#pragma unroll
-    for (int s = 0; s < S; ++s) {
-        const int slice = s0 + min(s, ns - 1), iz = slice % g.nz, b = slice / g.nz;
-        const float zc = ((float)iz - g.nz / 2.f) * g.dz + g.cz + g.dz / 2;
-        const int iv = (int)(zc / d.dv + d.off_v + d.nv / 2.f - 0.5f);
-        row_ok[s] = s < ns && iv >= 0 && iv < d.nv;
-        rows[s] = src + ((size_t)b * nview * d.nv + (row_ok[s] ? iv : 0)) * d.nu;
-        any_row |= row_ok[s];
-    }
-    const size_t vstride = (size_t)d.nv * d.nu;
-    const size_t tstride = (size_t)kPViews * stride;
-    const float hdx = g.dx / 2.0f, hdy = g.dy / 2.0f;
-    // x-layout: pixel centres (xs0 + k dx, ysx); y-layout: (xsy, ys0 + k dy)
-    const float xs0 = ((float)(tx0 + xl_col) - g.nx / 2.f) * g.dx + g.cx + hdx;
-    const float ysx = ((float)(ty0 + xl_row) - g.ny / 2.f) * g.dy + g.cy + hdy;
-    const float xsy = ((float)(tx0 + yl_col) - g.nx / 2.f) * g.dx + g.cx + hdx;
-    const float ys0 = ((float)(ty0 + yl_row) - g.ny / 2.f) * g.dy + g.cy + hdy;
-    const float jscale = -1.f / d.du, joff = -d.off_u + d.nu / 2.0f;
-    const float dso2 = dso * dso;
-    float ax[S][4], ay[S][4];
-#pragma unroll
-    for (int s = 0; s < S; ++s)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) ax[s][k] = ay[s][k] = 0.f;
-
-    img += blockIdx.z * part_elems;
-    const int vb = blockIdx.z * vper, ve = min(nview, vb + vper);
-    for (int v0 = vb; v0 < ve && any_row; v0 += kPViews) {
-        const int nvc = min(kPViews, ve - v0);
-        if (threadIdx.x < nvc) {
-            const int vi = threadIdx.x, view = v0 + vi;
-            double s, c;
-            sincos((double)deg[view], &s, &c);
-            // window: detector coordinates of the tile's corner edges
-            double xs[2] = {(tx0 - 0.5 * g.nx) * g.dx + g.cx, (tx0 + kPT - 0.5 * g.nx) * g.dx + g.cx};
-            double ys[2] = {(ty0 - 0.5 * g.ny) * g.dy + g.cy, (ty0 + kPT - 0.5 * g.ny) * g.dy + g.cy};
-            double jmin = 1e300, jmax = -1e300;
-            bool ok = true;
-            for (int a = 0; a < 2; ++a)
-                for (int q = 0; q < 2; ++q) {
-                    double ry = -xs[a] * s + ys[q] * c + dso;
-                    if (!(ry > 0)) ok = false;
-                    double j = -(atan((xs[a] * c + ys[q] * s) / ry) / d.du + (double)d.off_u) + 0.5 * d.nu;
-                    jmin = fmin(jmin, j);
-                    jmax = fmax(jmax, j);
-                }
-            int w0 = 0;
-            if (ok && isfinite(jmin) && isfinite(jmax)) {
-                w0 = (int)floor(jmin) - 2;
-                ok = ((int)ceil(jmax) + 2 - w0) <= win;
-            } else {
-                ok = false;
-            }
-            FanView V;
-            V.c = (float)c;
-            V.s = (float)s;
-            V.w0 = ok ? w0 : INT_MIN;
-            V.ym = ref_y_main(deg[view]) ? 1 : 0;
-            s_view[vi] = V;
-        }
-        __syncthreads();
-        for (int sv0 = warp; sv0 < S * nvc; sv0 += 8 * kStageBatch) {
-            WinItem<Tp> it[kStageBatch];
-#pragma unroll
-            for (int m = 0; m < kStageBatch; ++m) {
-                const int sv = sv0 + 8 * m;
-                const int s = sv / nvc, vi = sv - s * nvc;
-                const Tp* srow = rows[0];
-                bool rok = row_ok[0];
-#pragma unroll
-                for (int q = 1; q < S; ++q)
-                    if (s == q) {
-                        srow = rows[q];
-                        rok = row_ok[q];
-                    }
-                it[m].valid = sv < S * nvc;
-                it[m].w0 = s_view[vi].w0;
-                it[m].ok = it[m].valid && it[m].w0 != INT_MIN && rok;
-                it[m].T = s_tab + s * tstride + vi * stride;
-                it[m].row = srow + (size_t)(v0 + vi) * vstride;
-            }
-            stage_windows(it, win, d.nu, lane);
-        }
-        __syncthreads();
-        for (int vi = 0; vi < nvc; ++vi) {
-            const FanView V = s_view[vi];
-            const float2* T = s_tab + vi * stride;
-            const float fw0 = (float)V.w0 + 0.5f;  // window origin, shifted for the midpoint tables
-            // edge points p_k = p_0 + k * step, k = 0..4, rotated: (rx, ry)
-            float px, py, sx, sy;
-            if (V.ym) {
-                px = xs0 - hdx; py = ysx; sx = g.dx; sy = 0.f;
-            } else {
-                px = xsy; py = ys0 - hdy; sx = 0.f; sy = g.dy;
-            }
-            const float rx0 = px * V.c + py * V.s, ry0 = -px * V.s + py * V.c;
-            const float drx = sx * V.c + sy * V.s, dry = -sx * V.s + sy * V.c;
-            float j[5];
-#pragma unroll
-            for (int k = 0; k < 5; ++k) {
-                const float rx = fmaf((float)k, drx, rx0), ry = fmaf((float)k, dry, ry0);
-                j[k] = fmaf(atanf(__fdividef(rx, ry + dso)), jscale, joff);  // fast divide: a few ulp
-            }
-            float wgt[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                wgt[k] = 1.f;
-                if (fbp) {
-                    const float rxc = fmaf((float)k + 0.5f, drx, rx0), ryc = fmaf((float)k + 0.5f, dry, ry0);
-                    wgt[k] = __fdividef(dso2, rxc * rxc + (dso + ryc) * (dso + ryc));
-                }
-            }
-            float val[S][4];
-            if (V.w0 != INT_MIN) {
-                float f[S][5];
-#pragma unroll
-                for (int k = 0; k < 5; ++k) {
-                    const float xs = j[k] - fw0;
-                    const float tt = xs + kRoundMagic;
-                    const int i = __float_as_int(tt) - kRoundMagicBits;
-                    const float fr = xs - (tt - kRoundMagic);
-#pragma unroll
-                    for (int s = 0; s < S; ++s) {
-                        const float2 e = T[s * tstride + i];
-                        f[s][k] = fmaf(e.y, fr, e.x);
-                    }
-                }
-#pragma unroll
-                for (int s = 0; s < S; ++s)
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) val[s][k] = __fdividef(f[s][k + 1] - f[s][k], j[k + 1] - j[k]);
-            } else {
-#pragma unroll
-                for (int s = 0; s < S; ++s) {
-                    const Tp* grow = rows[s] + (size_t)(v0 + vi) * vstride;
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const float lo = fminf(j[k], j[k + 1]), hi = fmaxf(j[k], j[k + 1]);
-                        val[s][k] = row_ok[s] ? __fdividef(box_line(grow, 1, lo, hi, d.nu), hi - lo) : 0.f;
-                    }
-                }
-            }
-            if (V.ym) {
-#pragma unroll
-                for (int s = 0; s < S; ++s)
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) ax[s][k] = fmaf(val[s][k], wgt[k], ax[s][k]);
-            } else {
-#pragma unroll
-                for (int s = 0; s < S; ++s)
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) ay[s][k] = fmaf(val[s][k], wgt[k], ay[s][k]);
-            }
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int s = 0; s < S; ++s)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) s_acc[(s * kPT + xl_row) * (kPT + 1) + xl_col + k] = ax[s][k];
-    __syncthreads();
-    const int ix = tx0 + yl_col;
-#pragma unroll
-    for (int s = 0; s < S; ++s) {
-        if (s >= ns) continue;
-        const int slice = s0 + s, iz = slice % g.nz, b = slice / g.nz;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            int iy = ty0 + yl_row + k;
-            if (ix < g.nx && iy < g.ny) {
-                Tout* o = img + (((size_t)b * g.nz + iz) * g.ny + iy) * g.nx + ix;
-                float a = ay[s][k] + s_acc[(s * kPT + yl_row + k) * (kPT + 1) + yl_col];
-                if (accumulate) a += rdf(o);
-                stf(o, a);
-            }
-        }
-    }
-}
-
-// Staged window for the fast fan path: angular size of a 32x32 tile seen from
-// the nearest source position, in cells, or 0 if it does not fit.
-int fan_fast_window(const ctp_geometry& g) {
-    double hx = 0.5 * g.nx * g.dx, hy = 0.5 * g.ny * g.dy;
-    double rmax = sqrt((fabs(g.cx) + hx) * (fabs(g.cx) + hx) + (fabs(g.cy) + hy) * (fabs(g.cy) + hy));
-    double diag = kPT * sqrt((double)g.dx * g.dx + (double)g.dy * g.dy);
-    double near = (double)g.dso - rmax;
-    if (near <= diag) return 0;
-    double cells = 2 * atan(0.5 * diag / near) / fabs((double)g.du);
-    int win = (int)ceil(cells) + 8;
-    return win <= kPMaxWin ? win : 0;
-}
-
-// Staged window for the fast parallel path (cells), or 0 if it does not fit.
-int par_fast_window(const ctp_geometry& g) {
-    double du = fabs((double)g.du);
-    double w = ((kPT - 1) * ((double)g.dx + g.dy) + fmax(g.dx, g.dy)) / du;
-    int win = (int)ceil(w) + 8;
-    return win <= kPMaxWin ? win : 0;
-}
-
 // Staged window (cells) needed by a 16x16 tile, from a conservative bound on
 // the tile's projected size.  0 means "read the sinogram from global memory".
 int window_cells(const ctp_geometry& g, int geom) {
@@ -1960,6 +1391,17 @@ int build_table(float* base, const float* deg, const ctp_geometry& g, int geom, 
     return check_launch("dd_table_kernel");
 }
 
+// The z interpolation of every detector row lands exactly on its own slice.
+bool slices_match_rows(const ctp_geometry& g) {
+    if (g.nz != g.nv) return false;
+    for (size_t iv = 0; iv < g.nv; ++iv) {
+        double z = ((double)iv - (g.nv - 1) / 2.0 + g.off_v) * g.dv;
+        z = (z - g.cz) / g.dz + g.nz / 2.0 - 0.5;
+        if (fabs(z - (double)iv) > 1e-6) return false;
+    }
+    return true;
+}
+
 // The fast forward projector handles slices projected one to one onto
 // detector rows (nz == nv and the z interpolation of every row landing exactly
 // on its own slice, as for single-slice and matched stacks) and at most
@@ -1967,12 +1409,7 @@ int build_table(float* base, const float* deg, const ctp_geometry& g, int geom, 
 bool fp_fast_ok(const ctp_geometry& g, int& vgroup, int& nrows) {
     // also reached from the workspace query, before the geometry is validated
     if (g.nu == 0 || g.nview == 0 || g.nx == 0 || g.ny == 0 || g.nz == 0) return false;
-    if (g.nz != g.nv) return false;
-    for (size_t iv = 0; iv < g.nv; ++iv) {
-        double z = ((double)iv - (g.nv - 1) / 2.0 + g.off_v) * g.dv;
-        z = (z - g.cz) / g.dz + g.nz / 2.0 - 0.5;
-        if (fabs(z - (double)iv) > 1e-6) return false;
-    }
+    if (!slices_match_rows(g)) return false;
     int ipv = (int)((g.nu + 30) / 31);
     // views per CTA: the largest count whose edge groups fill the warps of one
     // of the compiled group counts (4, 8, 12, 16 per warp) with the least waste
@@ -2254,65 +1691,15 @@ int dd2d_nnz(unsigned long long* nnz_host, const float* deg, const ctp_geometry&
 
 namespace {
 
-// Sum of the view parts of a split back projection into the output.
-template <typename Tout>
-__global__ void bp_parts_sum_kernel(Tout* __restrict__ img, const float* __restrict__ parts, int nparts,
-                                    size_t elems, int accumulate) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < elems; i += (size_t)gridDim.x * blockDim.x) {
-        float a = accumulate ? rdf(img + i) : 0.f;
-        for (int q = 0; q < nparts; ++q) a += parts[(size_t)q * elems + i];
-        stf(img + i, a);
-    }
-}
-
-// View parts of a fast back projection whose grid (ctas) leaves SMs idle:
-// enough parts of whole kPViews chunks (at most 8) for about two CTAs per SM.
-// vper receives the views per part.
-int bp_view_parts(size_t ctas, int nview, int& vper) {
-    int sms = 148, dev = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int chunks = (nview + kPViews - 1) / kPViews;
-    if (chunks <= 0) {
-        vper = kPViews;
-        return 1;
-    }
-    int parts = 1;
-    if (ctas > 0 && ctas < (size_t)sms) {
-        parts = (int)std::min<size_t>(8, (2 * (size_t)sms + ctas - 1) / ctas);
-    } else if (ctas >= 2 * (size_t)sms && ctas < 6 * (size_t)sms) {
-        // A grid of one to three waves of equal CTAs (2 resident per SM: the
-        // fast kernels' registers and shared memory) whose last wave is far
-        // from full leaves SMs idle at the end: split the views into the
-        // parts (up to 8) that fill the waves best, summed by one more pass
-        // over the output.  Measured: the 4-slice 512^2 fan batch (512 CTAs,
-        // 1.7 waves) 1.60 -> 1.39 ms with 4 parts; the 16-slice parallel
-        // batch (1024 CTAs, 3.5 waves, whose tail is already spread over the
-        // SMs) unchanged with 2.
-        const double slots = 2.0 * sms;
-        auto fill = [&](int p) {
-            const double waves = (double)ctas * p / slots;
-            return waves / std::ceil(waves);
-        };
-        if (fill(1) < 0.95)
-            for (int p = 2; p <= 8; ++p)
-                if (fill(p) > fill(parts) + 0.02) parts = p;
-    }
-    parts = std::max(1, std::min(parts, chunks));
-    vper = ((chunks + parts - 1) / parts) * kPViews;
-    return (nview + vper - 1) / vper;
-}
-
-// CTAs of the fast back-projection grid (0 when the fast path does not apply).
-size_t bp_fast_ctas(const ctp_geometry& g, int geom) {
-    const size_t nslices = g.nbatch * g.nz;
-    const size_t tiles = ((g.nx + kPT - 1) / kPT) * ((g.ny + kPT - 1) / kPT);
-    if (geom == 0) {
-        if (fan_fast_window(g) <= 0) return 0;
-        return tiles * ((nslices + (nslices >= 2 ? 1 : 0)) / (nslices >= 2 ? 2 : 1));
-    }
-    if (par_fast_window(g) <= 0) return 0;
-    const size_t S = nslices >= 4 ? 4 : nslices >= 2 ? 2 : 1;
-    return tiles * ((nslices + S - 1) / S);
+// The tiled gather (dd2d_gather.cu) where it applies; branchless modes whose
+// operator differs from the box integral's take the general kernel (for a fan
+// beam with one detector row the operators coincide), and so do geometries
+// whose tiles do not fit its window.
+bool bp_gather(const ctp_geometry& g, int geom, int type, unsigned flags, GatherMode& mode) {
+    mode = (flags & CTP_FLAG_ADJOINT) ? kGatherAdjoint
+           : (type & (CTP_TYPE_FBP | CTP_TYPE_FORCE_FBP)) ? kGatherFbp : kGatherMean;
+    if (mode != kGatherAdjoint && (type & CTP_TYPE_BRANCHLESS) && (geom == 1 || g.nv > 1)) return false;
+    return gather_applies(g, geom, mode, slices_match_rows(g));
 }
 
 size_t bp_pre_bytes(const ctp_geometry& g, int geom, int type) {
@@ -2321,13 +1708,10 @@ size_t bp_pre_bytes(const ctp_geometry& g, int geom, int type) {
 }
 
 size_t bp_workspace(const ctp_geometry& g, int geom, int type, unsigned flags) {
+    GatherMode mode;
+    if (bp_gather(g, geom, type, flags, mode)) return gather_bytes(g, geom, mode);
     if (flags & CTP_FLAG_ADJOINT) return align_up(table_floats(g.nview, g.nu) * sizeof(float));
-    size_t need = bp_pre_bytes(g, geom, type);
-    const size_t ctas = bp_fast_ctas(g, geom);
-    int vper = 0;
-    const int parts = ctas ? bp_view_parts(ctas, (int)g.nview, vper) : 1;
-    if (parts > 1) need += align_up((size_t)parts * g.nbatch * g.nz * g.ny * g.nx * sizeof(float));
-    return need;
+    return bp_pre_bytes(g, geom, type);
 }
 
 template <typename Tin, typename Tout>
@@ -2362,55 +1746,9 @@ int launch_bp(void* img, const void* prj, const float* deg, const ctp_geometry& 
         return check_launch("dd2d_bp_adjoint_kernel");
     }
     int fbp = (type & (CTP_TYPE_FBP | CTP_TYPE_FORCE_FBP)) ? 1 : 0;
-    // branchless: the same operator as the box integral for a fan beam with
-    // one detector row; otherwise the general kernel in its branchless mode
     const int bl = (type & CTP_TYPE_BRANCHLESS) ? 1 : 0;
     size_t shm = (size_t)kBPViews * wl * 4 + kBPViews * 5 * 4;
     if (geom == 0) {
-        int fwin = (bl && g.nv > 1) ? 0 : fan_fast_window(g);
-        int tiles_f = (int)(((g.nx + kPT - 1) / kPT) * ((g.ny + kPT - 1) / kPT));
-        // two slices per CTA for stacks (shared edge mappings), one otherwise
-        const int nslices = (int)(g.nbatch * g.nz);
-        const int FS = nslices >= 2 ? 2 : 1;
-        size_t fshm = fan_fast_smem(fwin, FS);
-        // few tiles and slices: the views split into parts summed at the end
-        int vper = nview;
-        const int parts = fwin > 0 ? bp_view_parts(bp_fast_ctas(g, 0), nview, vper) : 1;
-        const size_t elems = g.nbatch * g.nz * g.ny * g.nx;
-        float* partial = reinterpret_cast<float*>(ws + bp_pre_bytes(g, geom, type));
-        dim3 fgrid((unsigned)tiles_f, (unsigned)((nslices + FS - 1) / FS), (unsigned)parts);
-        auto fan_fast = [&](auto k1, auto k2, auto kp1, auto kp2, const auto* srcp, int fbp_mode) {
-            if (parts == 1) {
-                auto k = FS == 2 ? k2 : k1;
-                cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fshm);
-                k<<<fgrid, 256, fshm, s>>>(mptr<Tout>(img), srcp, deg, nview, gr, dt, dso, fbp_mode, accumulate, fwin,
-                                           nslices, nview, (size_t)0);
-                return check_launch("dd2d_bp_fan_fast_kernel");
-            }
-            auto k = FS == 2 ? kp2 : kp1;
-            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fshm);
-            k<<<fgrid, 256, fshm, s>>>(partial, srcp, deg, nview, gr, dt, dso, fbp_mode, 0, fwin, nslices, vper,
-                                       elems);
-            int r = check_launch("dd2d_bp_fan_fast_kernel");
-            if (r) return r;
-            bp_parts_sum_kernel<Tout><<<(unsigned)std::min<size_t>((elems + 255) / 256, 148 * 8), 256, 0, s>>>(
-                mptr<Tout>(img), partial, parts, elems, accumulate);
-            return check_launch("bp_parts_sum_kernel");
-        };
-        if (fwin > 0 && !fbp) {
-            float* wprj = reinterpret_cast<float*>(ws);
-            size_t total = g.nbatch * g.nview * g.nv * g.nu;
-            fan_preweight_kernel<Tin><<<(unsigned)((total + 255) / 256), 256, 0, s>>>(wprj, cptr<Tin>(prj), deg,
-                                                                                    nview, dt, gr, total);
-            if ((rc = check_launch("fan_preweight_kernel"))) return rc;
-            return fan_fast(dd2d_bp_fan_fast_kernel<float, Tout, 1>, dd2d_bp_fan_fast_kernel<float, Tout, 2>,
-                            dd2d_bp_fan_fast_kernel<float, float, 1>, dd2d_bp_fan_fast_kernel<float, float, 2>,
-                            (const float*)wprj, 0);
-        }
-        if (fwin > 0)
-            return fan_fast(dd2d_bp_fan_fast_kernel<Tin, Tout, 1>, dd2d_bp_fan_fast_kernel<Tin, Tout, 2>,
-                            dd2d_bp_fan_fast_kernel<Tin, float, 1>, dd2d_bp_fan_fast_kernel<Tin, float, 2>,
-                            cptr<Tin>(prj), 1);
         if (!fbp) {
             float* wprj = reinterpret_cast<float*>(ws);
             size_t total = g.nbatch * g.nview * g.nv * g.nu;
@@ -2426,39 +1764,6 @@ int launch_bp(void* img, const void* prj, const float* deg, const ctp_geometry& 
                                                accumulate, win > 0 ? win : 0, bl);
         }
     } else {
-        int pwin = bl ? 0 : par_fast_window(g);
-        if (pwin > 0) {
-            int tiles_p = (int)(((g.nx + kPT - 1) / kPT) * ((g.ny + kPT - 1) / kPT));
-            // slices per CTA for stacks (shared per-view work): 4, 2 or 1
-            const int nslices = (int)(g.nbatch * g.nz);
-            const int S = nslices >= 4 ? 4 : nslices >= 2 ? 2 : 1;
-            size_t pshm = par_fast_smem(pwin, S);
-            // few tiles and slices: the views split into parts summed at the end
-            int vper = nview;
-            const int parts = bp_view_parts(bp_fast_ctas(g, 1), nview, vper);
-            const size_t elems = g.nbatch * g.nz * g.ny * g.nx;
-            float* partial = reinterpret_cast<float*>(ws + bp_pre_bytes(g, geom, type));
-            dim3 pg((unsigned)tiles_p, (unsigned)((nslices + S - 1) / S), (unsigned)parts);
-            auto par_fast = [&](auto kout, auto kpart) {
-                if (parts == 1) {
-                    cudaFuncSetAttribute(kout, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pshm);
-                    kout<<<pg, 256, pshm, s>>>(mptr<Tout>(img), cptr<Tin>(prj), deg, nview, gr, dt, fbp, accumulate,
-                                               pwin, nslices, nview, (size_t)0);
-                    return check_launch("dd2d_bp_par_fast_kernel");
-                }
-                cudaFuncSetAttribute(kpart, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pshm);
-                kpart<<<pg, 256, pshm, s>>>(partial, cptr<Tin>(prj), deg, nview, gr, dt, fbp, 0, pwin, nslices, vper,
-                                            elems);
-                int r = check_launch("dd2d_bp_par_fast_kernel");
-                if (r) return r;
-                bp_parts_sum_kernel<Tout><<<(unsigned)std::min<size_t>((elems + 255) / 256, 148 * 8), 256, 0, s>>>(
-                    mptr<Tout>(img), partial, parts, elems, accumulate);
-                return check_launch("bp_parts_sum_kernel");
-            };
-            if (S == 4) return par_fast(dd2d_bp_par_fast_kernel<Tin, Tout, 4>, dd2d_bp_par_fast_kernel<Tin, float, 4>);
-            if (S == 2) return par_fast(dd2d_bp_par_fast_kernel<Tin, Tout, 2>, dd2d_bp_par_fast_kernel<Tin, float, 2>);
-            return par_fast(dd2d_bp_par_fast_kernel<Tin, Tout, 1>, dd2d_bp_par_fast_kernel<Tin, float, 1>);
-        }
         auto k = dd2d_bp_parity_kernel<false, Tin, Tout>;
         k<<<grid, kTile * kTile, shm, s>>>(mptr<Tout>(img), cptr<Tin>(prj), deg, nview, gr, dt, dso, fbp,
                                            accumulate, win > 0 ? win : 0, bl);
@@ -2467,6 +1772,14 @@ int launch_bp(void* img, const void* prj, const float* deg, const ctp_geometry& 
 }
 
 }  // namespace
+
+// The storage combinations that the DD entries take: FP32 in and out, or 16-bit
+// in with the same type or FP32 out.
+static bool io_types_ok(unsigned flags) {
+    if (flags & CTP_FLAG_IN_BF16) return (flags & CTP_FLAG_OUT_BF16) || !(flags & CTP_FLAG_OUT_FP16);
+    if (flags & CTP_FLAG_IN_FP16) return (flags & CTP_FLAG_OUT_FP16) || !(flags & CTP_FLAG_OUT_BF16);
+    return !(flags & (CTP_FLAG_OUT_BF16 | CTP_FLAG_OUT_FP16));
+}
 
 size_t dd2d_bp_workspace(const ctp_geometry& g, int geom, int type, unsigned flags) {
     return bp_workspace(g, geom, type, flags);
@@ -2481,6 +1794,9 @@ int dd2d_bp(void* img, const void* prj, const float* deg, const ctp_geometry& g,
     if (rc) return rc;
     bool in16 = flags & (CTP_FLAG_IN_BF16 | CTP_FLAG_IN_FP16);
     bool out16 = flags & (CTP_FLAG_OUT_BF16 | CTP_FLAG_OUT_FP16);
+    GatherMode mode;
+    if (io_types_ok(flags) && bp_gather(g, geom, type, flags, mode))
+        return gather_bp(img, prj, deg, g, geom, mode, flags, scr.base(), s);
     if (!in16 && !out16) return launch_bp<float, float>(img, prj, deg, g, geom, type, flags, scr.base(), s);
     if ((flags & CTP_FLAG_IN_BF16) && (flags & CTP_FLAG_OUT_BF16))
         return launch_bp<__nv_bfloat16, __nv_bfloat16>(img, prj, deg, g, geom, type, flags, scr.base(), s);

@@ -1,0 +1,98 @@
+"""The tiled gather back projection (mean, FBP, adjoint) at the sizes where they can go wrong: ragged
+tiles, one to five slices per CTA group, more views than one list, wide tiles,
+flipped detectors and angles that are not numbers; against the FP64 oracle."""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+# A pixel adds one FP32 term per view (n <= 1100 here, in sums of at most 1024),
+# each the difference of two table entries of up to 60 cells: a few 2^-24 of 60
+# cells over a footprint of about one, at random over the views: below
+# 60 2^-23 / sqrt(40) = 1.1e-6 at 40 views and less with more.
+TOL = 3e-6
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _cuda():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+
+
+def dev(a):
+    return torch.tensor(np.ascontiguousarray(a, dtype=np.float32), device="cuda")
+
+
+def proj(geom, nx, ny, nu, nz=1, pixel=1.0, nview=40, **kw):
+    from cases import Proj
+
+    cell = kw.pop("cell", (1.35 if geom == "parallel" else 2.5) * np.hypot(nx, ny) * pixel / nu)
+    return Proj(nx=nx, ny=ny, nz=nz, dx=pixel, dy=pixel * kw.pop("aspect", 1.0), nu=nu, nv=nz, du=cell, dv=1.0,
+                nview=nview, **kw)
+
+
+def angles(nview, geom, start=0.013):
+    span = np.pi if geom == "parallel" else 2 * np.pi
+    return (start + np.arange(nview) * span / nview).astype(np.float32)
+
+
+def module(geom):
+    from ctprojector_b200.projector.cupy import fan_equiangular, parallel
+
+    return fan_equiangular if geom == "fan" else parallel
+
+
+def check(p, ang, geom, oracle, nbatch, modes=("mean", "fbp", "adjoint")):
+    rng = np.random.default_rng(p.nx + p.nu)
+    y = rng.uniform(0, 1, (nbatch, len(ang), p.nv, p.nu)).astype(np.float32)
+    for mode in modes:
+        kw = dict(is_fbp=mode == "fbp", adjoint=mode == "adjoint")
+        out = module(geom).distance_driven_bp(p, dev(y), dev(ang), **kw).cpu().numpy()
+        assert rel_l2(out, oracle.dd_bp(p, y, ang, geom, **kw)) <= TOL, mode
+
+
+@pytest.mark.parametrize("geom", ["fan", "parallel"])
+@pytest.mark.parametrize("nx,ny,nbatch", [(31, 33, 1), (32, 64, 2), (65, 29, 3), (40, 97, 5)])
+def test_tiles_and_slices(geom, nx, ny, nbatch, oracle):
+    p = proj(geom, nx, ny, 83, off_u=0.4, cx=1.0, cy=-2.0, aspect=1.2)
+    check(p, angles(40, geom), geom, oracle, nbatch)
+
+
+@pytest.mark.parametrize("geom", ["fan", "parallel"])
+def test_stack_with_rows(geom, oracle):
+    """nz = nv slices projected one to one."""
+    p = proj(geom, 34, 36, 60, nz=3)
+    check(p, angles(24, geom), geom, oracle, 2)
+
+
+@pytest.mark.parametrize("geom", ["fan", "parallel"])
+def test_more_views_than_one_list(geom, oracle):
+    p = proj(geom, 36, 20, 50, nview=1100)
+    check(p, angles(1100, geom), geom, oracle, 1)
+
+
+@pytest.mark.parametrize("pixel", [0.1, 6.0])
+def test_fan_small_and_wide_tiles(pixel, oracle):
+    """6 mm pixels: a tile spans more than the series of atan is used for."""
+    p = proj("fan", 40, 40, 70, pixel=pixel)
+    check(p, angles(36, "fan"), "fan", oracle, 2)
+
+
+@pytest.mark.parametrize("geom", ["fan", "parallel"])
+def test_flipped_detector(geom, oracle):
+    p = proj(geom, 33, 40, 64)
+    p.du = -p.du
+    check(p, angles(30, geom), geom, oracle, 2)
+
+
+@pytest.mark.parametrize("geom", ["fan", "parallel"])
+@pytest.mark.parametrize("kw", [{}, {"is_fbp": True}, {"adjoint": True}])
+def test_angle_that_is_not_a_number(geom, kw):
+    p = proj(geom, 40, 40, 64)
+    ang = angles(40, geom)
+    ang[7] = np.nan
+    out = module(geom).distance_driven_bp(p, torch.ones(2, 40, 1, 64, device="cuda"), dev(ang), **kw)
+    assert torch.isnan(out).all()
