@@ -191,37 +191,37 @@ __device__ __forceinline__ void stage_rows_per(const RowItem<Tp> (&it)[2], float
                 if (t1) reinterpret_cast<float2*>(t1)[k] = make_float2(v[1][q], step[1]);
             }
         }
-        return;
-    }
-#pragma unroll
-    for (int m = 0; m < 2; ++m) {
-        run[m] = 0.f;
-#pragma unroll
-        for (int q = 0; q < PER; ++q) run[m] += v[m][q];
-        incl[m] = run[m];
-    }
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1)
+    } else {
 #pragma unroll
         for (int m = 0; m < 2; ++m) {
-            const float t = __shfl_up_sync(0xffffffffu, incl[m], o);
-            if (lane >= o) incl[m] += t;
-        }
-    float b0 = incl[0] - run[0], b1 = incl[1] - run[1];
+            run[m] = 0.f;
 #pragma unroll
-    for (int q = 0; q < PER; ++q) {
-        const int k = k0 + q;
-        if (k <= win) {
-            const float m0 = fmaf(0.5f, v[0][q], b0), m1 = fmaf(0.5f, v[1][q], b1);
-            if constexpr (PAIR) {
-                reinterpret_cast<float4*>(t0)[k] = make_float4(m0, m1, v[0][q], v[1][q]);
-            } else {
-                reinterpret_cast<float2*>(t0)[k] = make_float2(m0, v[0][q]);
-                if (t1) reinterpret_cast<float2*>(t1)[k] = make_float2(m1, v[1][q]);
-            }
+            for (int q = 0; q < PER; ++q) run[m] += v[m][q];
+            incl[m] = run[m];
         }
-        b0 += v[0][q];
-        b1 += v[1][q];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                const float t = __shfl_up_sync(0xffffffffu, incl[m], o);
+                if (lane >= o) incl[m] += t;
+            }
+        float b0 = incl[0] - run[0], b1 = incl[1] - run[1];
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            const int k = k0 + q;
+            if (k <= win) {
+                const float m0 = fmaf(0.5f, v[0][q], b0), m1 = fmaf(0.5f, v[1][q], b1);
+                if constexpr (PAIR) {
+                    reinterpret_cast<float4*>(t0)[k] = make_float4(m0, m1, v[0][q], v[1][q]);
+                } else {
+                    reinterpret_cast<float2*>(t0)[k] = make_float2(m0, v[0][q]);
+                    if (t1) reinterpret_cast<float2*>(t1)[k] = make_float2(m1, v[1][q]);
+                }
+            }
+            b0 += v[0][q];
+            b1 += v[1][q];
+        }
     }
 }
 
@@ -515,7 +515,8 @@ __global__ void __launch_bounds__(256, (S == 4 ? 3 : 4)) gather_bp_kernel(const 
                             it[m].lw = lw ? lw + (size_t)view * d.nu : nullptr;
                             it[m].w0 = w0 != INT_MIN ? w0 : 0;
                         }
-                        stage_rows<true, MODE == kGatherPixel>(it, tab + (p * plane + vi * stride * L::kEntry) / 4, nullptr, A.win, d.nu, lane);
+                        stage_rows<true, MODE == kGatherPixel>(it, tab + (p * plane + vi * stride * L::kEntry) / 4, nullptr,
+                                                               A.win, d.nu, lane);
                     }
                 } else {
                     for (int i = warp * 2; i < n; i += 16) {
@@ -529,7 +530,8 @@ __global__ void __launch_bounds__(256, (S == 4 ? 3 : 4)) gather_bp_kernel(const 
                             it[m].w0 = w0 != INT_MIN ? w0 : 0;
                         }
                         float* t = tab + (size_t)i * stride * 2;
-                        stage_rows<false, MODE == kGatherPixel>(it, t, i + 1 < n ? t + stride * 2 : nullptr, A.win, d.nu, lane);
+                        stage_rows<false, MODE == kGatherPixel>(it, t, i + 1 < n ? t + stride * 2 : nullptr, A.win, d.nu,
+                                                                lane);
                     }
                 }
                 __syncthreads();

@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "ctp_common.cuh"
+#include "dd2d_gather.cuh"
 
 namespace ctp {
 
@@ -1194,10 +1195,29 @@ __global__ void pixel_bp_par_kernel(float* __restrict__ img, const float* __rest
     }
 }
 
+// The tiled gather (dd2d_gather.cu) for detectors of one row, when its scratch
+// (none, or the parts' volumes of a call of few tiles) can be had.
+int pixel_gather(float* img, const float* prj, const float* deg, const ctp_geometry& g, int geom, unsigned flags,
+                 cudaStream_t s, bool& done) {
+    done = false;
+    if (!gather_applies(g, geom, kGatherPixel, false)) return CTP_OK;
+    Scratch scr;
+    const size_t need = gather_bytes(g, geom, kGatherPixel);
+    if (need && scr.acquire(nullptr, 0, need, s)) {
+        cudaGetLastError();  // the general kernel needs none
+        return CTP_OK;
+    }
+    done = true;
+    return gather_bp(img, prj, deg, g, geom, kGatherPixel, flags, scr.base(), s);
+}
+
 }  // namespace
 
 int fbp_fan_bp(float* img, const float* prj, const float* deg, const ctp_geometry& g, unsigned flags,
                cudaStream_t s) {
+    bool done;
+    int rc = pixel_gather(img, prj, deg, g, 0, flags, s, done);
+    if (done) return rc;
     int zb = (int)((g.nz + kFbpZ - 1) / kFbpZ);
     dim3 grid((unsigned)((g.nx + 31) / 32), (unsigned)((g.ny + 7) / 8), (unsigned)(g.nbatch * zb));
     fbp_fan_bp_kernel<<<grid, 256, 0, s>>>(img, prj, deg, (int)g.nview, make_grid(g), make_det(g), g.dso,
@@ -1207,6 +1227,9 @@ int fbp_fan_bp(float* img, const float* prj, const float* deg, const ctp_geometr
 
 int pixel_bp_parallel(float* img, const float* prj, const float* deg, const ctp_geometry& g, unsigned flags,
                       cudaStream_t s) {
+    bool done;
+    int rc = pixel_gather(img, prj, deg, g, 1, flags, s, done);
+    if (done) return rc;
     int zb = (int)((g.nz + kFbpZ - 1) / kFbpZ);
     dim3 grid((unsigned)((g.nx + 31) / 32), (unsigned)((g.ny + 7) / 8), (unsigned)(g.nbatch * zb));
     pixel_bp_par_kernel<<<grid, 256, 0, s>>>(img, prj, deg, (int)g.nview, make_grid(g), make_det(g),

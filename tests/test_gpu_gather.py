@@ -1,5 +1,5 @@
-"""The tiled gather back projection (mean, FBP, adjoint) at the sizes where they can go wrong: ragged
-tiles, one to five slices per CTA group, more views than one list, wide tiles,
+"""The tiled gather back projection (mean, FBP, adjoint, pixel-driven) at the
+sizes where it can go wrong: ragged tiles, one to five slices per CTA group, more views than one list, wide tiles,
 flipped detectors and angles that are not numbers; against the FP64 oracle."""
 import numpy as np
 import pytest
@@ -96,3 +96,22 @@ def test_angle_that_is_not_a_number(geom, kw):
     ang[7] = np.nan
     out = module(geom).distance_driven_bp(p, torch.ones(2, 40, 1, 64, device="cuda"), dev(ang), **kw)
     assert torch.isnan(out).all()
+
+
+@pytest.mark.parametrize("nbatch", [1, 2, 4])
+@pytest.mark.parametrize("geom", ["fan", "parallel"])
+def test_pixel_driven(geom, nbatch, oracle):
+    """Detectors narrower and wider than the grid (pixels off the detector add nothing)."""
+    for width in (0.6, 1.3):
+        p = proj(geom, 45, 38, 61, cell=width * (2.4 if geom == "fan" else 1.0) * 45 / 61)
+        ang = angles(50, geom)
+        y = np.random.default_rng(nbatch).uniform(0, 1, (nbatch, 50, 1, 61)).astype(np.float32)
+        if geom == "fan":
+            out, ref = module(geom).fbp_bp(p, dev(y), dev(ang)), oracle.fbp_bp(p, y, ang)
+        else:
+            out, ref = module(geom).pixel_driven_bp(p, dev(y), dev(ang)), oracle.pixel_bp_parallel(p, y, ang)
+        # a pixel whose centre falls within rounding of the detector's end may
+        # count or not: one cell of one view
+        bad = np.abs(out.cpu().numpy() - ref) > 1e-4 * np.abs(ref).max()
+        assert bad.sum() <= 2
+        assert rel_l2(np.where(bad, ref, out.cpu().numpy()), ref) <= TOL
