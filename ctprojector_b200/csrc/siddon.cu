@@ -17,7 +17,11 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include <algorithm>
+#include <type_traits>
+
 #include "ctp_common.cuh"
+#include "siddon_columns.cuh"
 
 namespace ctp {
 
@@ -173,17 +177,31 @@ __device__ __forceinline__ void walk(const Ray& R, const Grid& g, F&& emit) {
     walk_strided<IdxT>(R, g, (IdxT)1, (IdxT)g.nx, (IdxT)g.nx * g.ny, emit);
 }
 
+// The view and batch item of a block: all nview views (rest null), or those
+// that the column kernels left, rest[1 .. rest[0]] (view_setup_kernel); false
+// for the blocks past them.
+__device__ __forceinline__ bool block_view(const int* __restrict__ rest, int nview, int& view, int& b) {
+    view = blockIdx.z % nview;
+    b = blockIdx.z / nview;
+    if (!rest) return true;
+    if (view >= rest[0]) return false;
+    view = rest[1 + view];
+    return true;
+}
+
 // Five CTAs per SM (48 registers): the walk is latency-bound on its
 // dependent loads, and the extra warps hide ~1% more of it.
 template <typename Tin, typename Tout, typename IdxT>
 __global__ void __launch_bounds__(256, 5) siddon_fp_kernel(Tout* __restrict__ prj, const Tin* __restrict__ img,
                                                         const float* __restrict__ dc, const float* __restrict__ du_,
                                                         const float* __restrict__ dv_, const float* __restrict__ sr,
-                                                        int nview, Grid g, Det d, int accumulate) {
+                                                        const int* __restrict__ rest, int nview, Grid g, Det d,
+                                                        int accumulate) {
     int iu = blockIdx.x * 32 + (threadIdx.x & 31);
     int iv = blockIdx.y * 8 + (threadIdx.x >> 5);
-    int view = blockIdx.z % nview, b = blockIdx.z / nview;
     if (iu >= d.nu || iv >= d.nv) return;
+    int view, b;
+    if (!block_view(rest, nview, view, b)) return;
     double src[3], dst[3];
     ray_ends(src, dst, view, iu, iv, dc, du_, dv_, sr, g, d);
     Ray R = init_ray(src, dst, g);
@@ -217,11 +235,13 @@ template <typename Tin, typename IdxT>
 __global__ void __launch_bounds__(256) siddon_bp_kernel(float* __restrict__ img, float* __restrict__ imgT,
                                                         const Tin* __restrict__ prj, const float* __restrict__ dc,
                                                         const float* __restrict__ du_, const float* __restrict__ dv_,
-                                                        const float* __restrict__ sr, int nview, Grid g, Det d) {
+                                                        const float* __restrict__ sr, const int* __restrict__ rest,
+                                                        int nview, Grid g, Det d) {
     int iu = blockIdx.x * 32 + (threadIdx.x & 31);
     int iv = blockIdx.y * 8 + (threadIdx.x >> 5);
-    int view = blockIdx.z % nview, b = blockIdx.z / nview;
     if (iu >= d.nu || iv >= d.nv) return;
+    int view, b;
+    if (!block_view(rest, nview, view, b)) return;
     float p = ldf(prj + (((size_t)b * nview + view) * d.nv + iv) * d.nu + iu);
     if (p == 0.f) return;
     double src[3], dst[3];
@@ -237,21 +257,34 @@ __global__ void __launch_bounds__(256) siddon_bp_kernel(float* __restrict__ img,
         walk<IdxT>(R, g, [&](IdxT idx, float len) { atomicAdd(vol + idx, p * len); });
 }
 
-// img[b][z][y][x] += imgT[b][z][x][y], through 32x32 shared tiles.
+// img[b][z][y][x] += imgT[b][z][x][y], through 32x32 shared tiles; nothing
+// when the column kernels left no view (rest[0] = 0).
 __global__ void __launch_bounds__(256) add_transposed_kernel(float* __restrict__ img, const float* __restrict__ imgT,
-                                                             int nx, int ny) {
+                                                             int nx, int ny, const int* __restrict__ rest,
+                                                             int planes) {
     __shared__ float t[32][33];
-    const size_t plane = (size_t)blockIdx.z * nx * ny;
+    if (rest && rest[0] == 0) return;
     const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
-    for (int k = threadIdx.y; k < 32; k += 8) {  // read rows of imgT: x fixed, y contiguous
-        const int x = x0 + k, y = y0 + threadIdx.x;
-        if (x < nx && y < ny) t[k][threadIdx.x] = imgT[plane + (size_t)x * ny + y];
+    for (int pl = blockIdx.z; pl < planes; pl += gridDim.z) {
+        const size_t plane = (size_t)pl * nx * ny;
+        __syncthreads();
+        for (int k = threadIdx.y; k < 32; k += 8) {  // read rows of imgT: x fixed, y contiguous
+            const int x = x0 + k, y = y0 + threadIdx.x;
+            if (x < nx && y < ny) t[k][threadIdx.x] = imgT[plane + (size_t)x * ny + y];
+        }
+        __syncthreads();
+        for (int k = threadIdx.y; k < 32; k += 8) {
+            const int y = y0 + k, x = x0 + threadIdx.x;
+            if (x < nx && y < ny) img[plane + (size_t)y * nx + x] += t[threadIdx.x][k];
+        }
     }
-    __syncthreads();
-    for (int k = threadIdx.y; k < 32; k += 8) {
-        const int y = y0 + k, x = x0 + threadIdx.x;
-        if (x < nx && y < ny) img[plane + (size_t)y * nx + x] += t[threadIdx.x][k];
-    }
+}
+
+// Zeroes the scatter copy when the column kernels left views.
+__global__ void __launch_bounds__(256) zero_if_rest_kernel(float* __restrict__ p, size_t n,
+                                                           const int* __restrict__ rest) {
+    if (rest[0] == 0) return;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) p[i] = 0.f;
 }
 
 __global__ void __launch_bounds__(256) siddon_count_kernel(unsigned long long* __restrict__ count,
@@ -360,38 +393,37 @@ bool small_volume(const ctp_geometry& g) { return (unsigned long long)g.nx * g.n
 
 template <typename IdxT>
 int launch_siddon_fp(void* prj, const void* img, const float* dc, const float* du_, const float* dv_, const float* sr,
-                     const ctp_geometry& g, unsigned flags, cudaStream_t s) {
+                     const int* rest, const ctp_geometry& g, unsigned flags, cudaStream_t s) {
     int acc = (flags & CTP_FLAG_ZERO_OUT) ? 0 : 1;
     dim3 grid = ray_grid(g, g.nbatch);
     Grid gr = make_grid(g);
     Det dt = make_det(g);
     int nv = (int)g.nview;
+    auto go = [&](auto* out, auto* in) {
+        using Tout = std::remove_pointer_t<decltype(out)>;
+        using Tin = std::remove_pointer_t<decltype(in)>;
+        siddon_fp_kernel<Tin, Tout, IdxT><<<grid, 256, 0, s>>>((Tout*)prj, (const Tin*)img, dc, du_, dv_, sr, rest, nv,
+                                                               gr, dt, acc);
+    };
+    __nv_bfloat16* bf = nullptr;
+    __half* hf = nullptr;
+    float* f32 = nullptr;
     if (flags & CTP_FLAG_IN_BF16) {
-        if (flags & CTP_FLAG_OUT_BF16)
-            siddon_fp_kernel<__nv_bfloat16, __nv_bfloat16, IdxT><<<grid, 256, 0, s>>>(
-                (__nv_bfloat16*)prj, (const __nv_bfloat16*)img, dc, du_, dv_, sr, nv, gr, dt, acc);
-        else
-            siddon_fp_kernel<__nv_bfloat16, float, IdxT><<<grid, 256, 0, s>>>(
-                (float*)prj, (const __nv_bfloat16*)img, dc, du_, dv_, sr, nv, gr, dt, acc);
+        if (flags & CTP_FLAG_OUT_BF16) go(bf, bf);
+        else go(f32, bf);
     } else if (flags & CTP_FLAG_IN_FP16) {
-        if (flags & CTP_FLAG_OUT_FP16)
-            siddon_fp_kernel<__half, __half, IdxT><<<grid, 256, 0, s>>>((__half*)prj, (const __half*)img, dc, du_, dv_,
-                                                                        sr, nv, gr, dt, acc);
-        else
-            siddon_fp_kernel<__half, float, IdxT><<<grid, 256, 0, s>>>((float*)prj, (const __half*)img, dc, du_, dv_,
-                                                                       sr, nv, gr, dt, acc);
+        if (flags & CTP_FLAG_OUT_FP16) go(hf, hf);
+        else go(f32, hf);
     } else {
-        if (flags & (CTP_FLAG_OUT_BF16 | CTP_FLAG_OUT_FP16))
-            return set_error(CTP_ERR_UNSUPPORTED, "siddon_fp: FP32 input with 16-bit output is not supported");
-        siddon_fp_kernel<float, float, IdxT><<<grid, 256, 0, s>>>((float*)prj, (const float*)img, dc, du_, dv_, sr,
-                                                                  nv, gr, dt, acc);
+        go(f32, f32);
     }
     return check_launch("siddon_fp_kernel");
 }
 
+// rest: the views that the column kernels left (null: every view).
 template <typename IdxT>
 int launch_siddon_bp(void* img, const void* prj, const float* dc, const float* du_, const float* dv_,
-                     const float* sr, const ctp_geometry& g, unsigned flags, cudaStream_t s) {
+                     const float* sr, const int* rest, const ctp_geometry& g, unsigned flags, cudaStream_t s) {
     dim3 grid = ray_grid(g, g.nbatch);
     // the transposed scatter target (zeroed), when the scratch can be had
     const size_t vox = g.nbatch * g.nz * g.ny * g.nx;
@@ -399,26 +431,34 @@ int launch_siddon_bp(void* img, const void* prj, const float* dc, const float* d
     float* imgT = nullptr;
     if (!scr.acquire(nullptr, 0, vox * sizeof(float), s)) {
         imgT = reinterpret_cast<float*>(scr.base());
-        cudaError_t e = cudaMemsetAsync(imgT, 0, vox * sizeof(float), s);
-        if (e != cudaSuccess) return set_error((int)e, "siddon_bp memset: %s", cudaGetErrorString(e));
+        if (rest) {
+            zero_if_rest_kernel<<<148 * 4, 256, 0, s>>>(imgT, vox, rest);
+            int rc = check_launch("zero_if_rest_kernel");
+            if (rc) return rc;
+        } else {
+            cudaError_t e = cudaMemsetAsync(imgT, 0, vox * sizeof(float), s);
+            if (e != cudaSuccess) return set_error((int)e, "siddon_bp memset: %s", cudaGetErrorString(e));
+        }
     } else {
         cudaGetLastError();  // fall back to the plain layout
     }
+    const int nv = (int)g.nview;
     if (flags & CTP_FLAG_IN_BF16)
         siddon_bp_kernel<__nv_bfloat16, IdxT><<<grid, 256, 0, s>>>((float*)img, imgT, (const __nv_bfloat16*)prj, dc,
-                                                                   du_, dv_, sr, (int)g.nview, make_grid(g),
+                                                                   du_, dv_, sr, rest, nv, make_grid(g),
                                                                    make_det(g));
     else if (flags & CTP_FLAG_IN_FP16)
         siddon_bp_kernel<__half, IdxT><<<grid, 256, 0, s>>>((float*)img, imgT, (const __half*)prj, dc, du_, dv_, sr,
-                                                            (int)g.nview, make_grid(g), make_det(g));
+                                                            rest, nv, make_grid(g), make_det(g));
     else
         siddon_bp_kernel<float, IdxT><<<grid, 256, 0, s>>>((float*)img, imgT, (const float*)prj, dc, du_, dv_, sr,
-                                                           (int)g.nview, make_grid(g), make_det(g));
+                                                           rest, nv, make_grid(g), make_det(g));
     int rc = check_launch("siddon_bp_kernel");
     if (rc || !imgT) return rc;
+    const unsigned planes = (unsigned)(g.nbatch * g.nz);
     add_transposed_kernel<<<dim3((unsigned)((g.nx + 31) / 32), (unsigned)((g.ny + 31) / 32),
-                                 (unsigned)(g.nbatch * g.nz)),
-                            dim3(32, 8), 0, s>>>((float*)img, imgT, (int)g.nx, (int)g.ny);
+                                 rest ? std::min(planes, 8u) : planes),
+                            dim3(32, 8), 0, s>>>((float*)img, imgT, (int)g.nx, (int)g.ny, rest, (int)planes);
     return check_launch("add_transposed_kernel");
 }
 
@@ -426,8 +466,23 @@ int launch_siddon_bp(void* img, const void* prj, const float* dc, const float* d
 
 int siddon_fp(void* prj, const void* img, const float* dc, const float* du_, const float* dv_, const float* sr,
               const ctp_geometry& g, unsigned flags, cudaStream_t s) {
-    return small_volume(g) ? launch_siddon_fp<int>(prj, img, dc, du_, dv_, sr, g, flags, s)
-                           : launch_siddon_fp<long long>(prj, img, dc, du_, dv_, sr, g, flags, s);
+    if (!(flags & (CTP_FLAG_IN_BF16 | CTP_FLAG_IN_FP16)) && (flags & (CTP_FLAG_OUT_BF16 | CTP_FLAG_OUT_FP16)))
+        return set_error(CTP_ERR_UNSUPPORTED, "siddon_fp: FP32 input with 16-bit output is not supported");
+    auto rays = [&](const int* rest) {
+        return small_volume(g) ? launch_siddon_fp<int>(prj, img, dc, du_, dv_, sr, rest, g, flags, s)
+                               : launch_siddon_fp<long long>(prj, img, dc, du_, dv_, sr, rest, g, flags, s);
+    };
+    // upright views column by column, when the scratch can be had; the others ray by ray
+    if (columns_fp_applies(g)) {
+        Scratch scr;
+        if (!scr.acquire(nullptr, 0, columns_fp_bytes(g, flags), s)) {
+            ColumnsPlan plan;
+            int rc = columns_fp(plan, scr.base(), prj, img, dc, du_, dv_, sr, g, flags, s);
+            return rc ? rc : rays(plan.rest);
+        }
+        cudaGetLastError();
+    }
+    return rays(nullptr);
 }
 
 int siddon_bp(void* img, const void* prj, const float* dc, const float* du_, const float* dv_, const float* sr,
@@ -438,8 +493,20 @@ int siddon_bp(void* img, const void* prj, const float* dc, const float* du_, con
         cudaError_t e = cudaMemsetAsync(img, 0, g.nbatch * g.nz * g.ny * g.nx * sizeof(float), s);
         if (e != cudaSuccess) return set_error((int)e, "siddon_bp memset: %s", cudaGetErrorString(e));
     }
-    return small_volume(g) ? launch_siddon_bp<int>(img, prj, dc, du_, dv_, sr, g, flags, s)
-                           : launch_siddon_bp<long long>(img, prj, dc, du_, dv_, sr, g, flags, s);
+    auto rays = [&](const int* rest) {
+        return small_volume(g) ? launch_siddon_bp<int>(img, prj, dc, du_, dv_, sr, rest, g, flags, s)
+                               : launch_siddon_bp<long long>(img, prj, dc, du_, dv_, sr, rest, g, flags, s);
+    };
+    if (columns_bp_applies(g)) {
+        Scratch scr;
+        if (!scr.acquire(nullptr, 0, columns_bp_bytes(g), s)) {
+            ColumnsPlan plan;
+            int rc = columns_bp(plan, scr.base(), (float*)img, prj, dc, du_, dv_, sr, g, flags, s);
+            return rc ? rc : rays(plan.rest);
+        }
+        cudaGetLastError();
+    }
+    return rays(nullptr);
 }
 
 int siddon_nnz(unsigned long long* nnz_host, const float* dc, const float* du_, const float* dv_, const float* sr,
@@ -499,7 +566,7 @@ int siddon_fan_bp(float* img, const float* prj, const float* deg, const ctp_geom
     if (rc || !imgT) return rc;
     add_transposed_kernel<<<dim3((unsigned)((g.nx + 31) / 32), (unsigned)((g.ny + 31) / 32),
                                  (unsigned)(g.nbatch * g.nz)),
-                            dim3(32, 8), 0, s>>>(img, imgT, (int)g.nx, (int)g.ny);
+                            dim3(32, 8), 0, s>>>(img, imgT, (int)g.nx, (int)g.ny, nullptr, (int)(g.nbatch * g.nz));
     return check_launch("add_transposed_kernel");
 }
 

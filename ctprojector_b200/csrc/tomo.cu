@@ -14,9 +14,9 @@
 // into the workspace.  The rectangles' two sides are separable, so threads
 // share the work along y: 64 x 256 x 512 voxels, 25 views of 1024 x 512 cells of
 // 0.25 mm, forward and back 4.55 -> 1.58 ms against one rectangle per thread and
-// plane (or view); both kernels are bound by instruction issue and the L1.  Unlike the reference, every batch item reads its own
-// weighted projections (the reference reads item 0's for all items,
-// distanceDriven3DBoxInt.cu:257-259).
+// plane (or view); both kernels are bound by instruction issue and the L1.
+// Unlike the reference, every batch item reads its own weighted projections
+// (the reference reads item 0's for all items, distanceDriven3DBoxInt.cu:257-259).
 #include <cuda_runtime.h>
 #include <math.h>
 

@@ -1,0 +1,116 @@
+"""Column-wise Siddon cone projectors (upright views) at the sizes where they
+can go wrong: rows around the 16-lane and 64-row passes, z around the 32-voxel
+chunks, detector windows wider than the staged one, flipped axes, and views
+left to the ray-driven kernels."""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+# A ray or a voxel adds at most n = 1000 FP32 terms here, each rounded to 2^-24
+# of the partial sum: sqrt(n) 2^-24 = 1.9e-6 for random signs, and a segment
+# split at a z plane is off by up to 2^-24 of z (128 voxels) over its z rise
+# (about 1% of the segments, less than 1e-4 of a voxel each).
+TOL = 4e-6
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _cuda():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+
+
+def scan(nx, ny, nz, nu, nv, nview=13, pixel=3.0, dz=2.0, cell=None, row=None, **kw):
+    from cases import Proj
+
+    cell = cell if cell is not None else 1.9 * pixel * max(nx, ny) / nu
+    row = row if row is not None else 1.9 * dz * nz / nv
+    return Proj(nx=nx, ny=ny, nz=nz, dx=pixel, dy=pixel, dz=dz, nu=nu, nv=nv, du=cell, dv=row, nview=nview, **kw)
+
+
+def helix(p, feed=0.0):
+    from ctprojector_b200 import synthetic as S
+
+    return list(S.helical(p.nview, 1.0, p.dso, p.dsd, feed))
+
+
+def check(p, geo, oracle, nbatch=1, tol=TOL):
+    from ctprojector_b200.projector.cupy import cone
+
+    rng = np.random.default_rng(p.nu + p.nv)
+    img = rng.uniform(0, 1, (nbatch, p.nz, p.ny, p.nx)).astype(np.float32)
+    prj = rng.uniform(-0.5, 1, (nbatch, p.nview, p.nv, p.nu)).astype(np.float32)
+    dev = [torch.tensor(a, device="cuda") for a in geo]
+    fp = cone.siddon_fp_arbitrary(p, torch.tensor(img, device="cuda"), *dev).cpu().numpy()
+    bp = cone.siddon_bp_arbitrary(p, torch.tensor(prj, device="cuda"), *dev).cpu().numpy()
+    assert rel_l2(fp, oracle.siddon_fp(p, img, *geo)) <= tol
+    assert rel_l2(bp, oracle.siddon_bp(p, prj, *geo)) <= tol
+
+
+@pytest.mark.parametrize("nz,nv", [(4, 8), (16, 17), (31, 16), (32, 33), (33, 48), (40, 65), (65, 130)])
+def test_rows_and_slices(nz, nv, oracle):
+    p = scan(37, 29, nz, 53, nv)
+    check(p, helix(p, feed=0.4 * nz * p.dz), oracle, nbatch=2)
+
+
+@pytest.mark.parametrize("nx,ny,nu", [(16, 16, 16), (17, 47, 33), (64, 15, 129), (48, 48, 400)])
+def test_grid_and_detector_sizes(nx, ny, nu, oracle):
+    """400 cells over 48 pixels: windows wider than the staged one."""
+    p = scan(nx, ny, 12, nu, 12, off_u=0.3, off_v=-0.7, cx=1.5, cy=-2.0, cz=0.6)
+    check(p, helix(p), oracle)
+
+
+@pytest.mark.parametrize("row", [0.2, 30.0])
+def test_fine_and_coarse_rows(row, oracle):
+    """0.2 mm rows: many through one plane inside a pixel, and more than the staged rows per chunk."""
+    p = scan(24, 24, 36, 40, 150 if row < 1 else 9, dz=1.0, row=row)
+    check(p, helix(p), oracle)
+
+
+@pytest.mark.parametrize("flip", ["u", "v", "uv"])
+def test_flipped_detector_axes(flip, oracle):
+    p = scan(33, 40, 20, 50, 24)
+    geo = helix(p, feed=10.0)
+    if "u" in flip:
+        geo[1] = -geo[1]
+    if "v" in flip:
+        geo[2] = -geo[2]
+    check(p, geo, oracle)
+
+
+def test_tilted_views_among_upright_ones(oracle):
+    """Every third view tilts its detector: the ray-driven kernels take those."""
+    p = scan(33, 28, 18, 44, 21)
+    geo = helix(p, feed=8.0)
+    a = 0.15
+    for k in range(0, p.nview, 3):
+        u, v = geo[1][k].copy(), geo[2][k].copy()
+        geo[1][k] = np.cos(a) * u + np.sin(a) * v
+        geo[2][k] = np.cos(a) * v - np.sin(a) * u
+    check(p, geo, oracle)
+
+
+def test_infinite_and_nan_cells_stay_on_their_rays(oracle):
+    """A view with an infinity or NaN is scattered ray by ray: the voxels that
+    its ray does not cross are those of the projections without it."""
+    from ctprojector_b200.projector.cupy import cone
+
+    p = scan(24, 24, 12, 30, 14)
+    geo = helix(p)
+    dev = [torch.tensor(a, device="cuda") for a in geo]
+    prj = np.random.default_rng(3).uniform(0, 1, (1, p.nview, p.nv, p.nu)).astype(np.float32)
+    bad = prj.copy()
+    bad[0, 4, 6, 15] = np.nan
+    bad[0, 7, 3, 11] = np.inf
+    mark = np.zeros_like(prj)
+    mark[0, 4, 6, 15] = mark[0, 7, 3, 11] = 1
+    chord = oracle.siddon_bp(p, mark, *geo)
+    out = cone.siddon_bp_arbitrary(p, torch.tensor(bad, device="cuda"), *dev).cpu().numpy()
+    ref = oracle.siddon_bp(p, np.where(mark > 0, 0, prj).astype(np.float32), *geo)
+    assert not np.isfinite(out[chord > 1e-3]).any()
+    clean = (chord == 0) & np.isfinite(out)
+    assert (chord == 0).sum() - clean.sum() <= 2  # a ray may graze one voxel more or less
+    assert rel_l2(out[clean], ref[clean]) <= TOL
