@@ -18,10 +18,11 @@
 //    cell.  The forward projector
 //    and its exact transpose read the same FP32 table entries, so both see
 //    bit-identical footprints.
-//  * Forward projection: one thread per ray, rows read with coalesced loads
-//    (adjacent threads = adjacent cells).  Views traced along x read a
-//    transposed copy of the image so that those walks are row reads too.
-//  * Back projection is a gather (no atomics): a CTA owns a 16x16 pixel tile,
+//  * Forward projection streams the image's line tables through shared memory
+//    (dd2d_fp_stream_kernel).  Views traced along x read a transposed copy of
+//    the image so that those walks are row reads too.
+//  * Back projection is a gather (no atomics), tiled in dd2d_gather.cu.  The
+//    kernels here take what it does not: a CTA owns a 16x16 pixel tile,
 //    streams chunks of views and stages, per view, only the window of
 //    detector cells that the tile projects onto in shared memory.  Two modes:
 //      - reference parity: the normalised detector-space box integral of
@@ -128,12 +129,69 @@ __device__ void edge_ray(int geom, double th, int j, const Grid& g, const Det& d
     ey = (ey - g.cy) / g.dy + 0.5 * g.ny;
 }
 
-// hard != 0: the branchless tracer's weights (distanceDriven2DBranchless.cu:
-// 68-118): the main axis alone, chosen by |__cosf| > |__sinf| as there.
+// Blend weight of the row (y main axis) sweep.  hard != 0: the branchless
+// tracer's weights (distanceDriven2DBranchless.cu:68-118): the main axis alone,
+// chosen by |__cosf| > |__sinf| as there.
+__device__ __forceinline__ float view_weight(float th, int hard) {
+    if (hard) return fabsf(__cosf(th)) > fabsf(__sinf(th)) ? 1.f : 0.f;
+    double s, c;
+    sincos((double)th, &s, &c);
+    const double r = (fabs(c) - fabs(s) + kDDMarginD) / (2 * kDDMarginD);
+    return (float)(r < 0 ? 0.0 : (r > 1 ? 1.0 : r));
+}
+
+// The views in the order the streamed forward projector takes them: those of
+// the blend band (0 < weight < 1), which sweep both orientations and so take
+// about twice as long, first, then the others, each in their original order
+// (a stable partition).  The launch dispatches view groups in this order, so
+// its longest CTAs start in the first wave instead of trailing the last.
+// One block; ballots and per-warp counts give each view its position.  Its own
+// launch cost a 256 x 256 fan slice, 360 views, 3% of the pair (217 -> 211 us).
+__device__ void order_blend_first(int* __restrict__ order, const float* __restrict__ deg, int nview, int hard) {
+    __shared__ int s_cnt[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    auto in_band = [&](int v) {
+        if (v >= nview) return false;
+        const float w = view_weight(deg[v], hard);
+        return w > 0.f && w < 1.f;
+    };
+    int nband = 0;
+    for (int t0 = 0; t0 < nview; t0 += blockDim.x) nband += __syncthreads_count(in_band(t0 + threadIdx.x));
+    int placed_band = 0, placed_rest = 0;
+    for (int t0 = 0; t0 < nview; t0 += blockDim.x) {
+        const int v = t0 + threadIdx.x;
+        const bool in = v < nview, band = in_band(v);
+        const unsigned mb = __ballot_sync(0xffffffffu, band), mi = __ballot_sync(0xffffffffu, in);
+        const unsigned below = (1u << lane) - 1u;
+        if (lane == 0) s_cnt[warp] = __popc(mb) | (__popc(mi) << 16);
+        __syncthreads();
+        int band_before = __popc(mb & below), all_before = __popc(mi & below), tile_band = 0, tile_all = 0;
+        for (int w = 0; w < nw; ++w) {
+            const int c = s_cnt[w];
+            if (w < warp) {
+                band_before += c & 0xffff;
+                all_before += c >> 16;
+            }
+            tile_band += c & 0xffff;
+            tile_all += c >> 16;
+        }
+        if (in)
+            order[band ? placed_band + band_before : nband + placed_rest + (all_before - band_before)] = v;
+        placed_band += tile_band;
+        placed_rest += tile_all - tile_band;
+        __syncthreads();
+    }
+}
+
+// order (may be null): the last block of the first view orders the views.
 __global__ void dd_table_kernel(DDTabW t, const float* __restrict__ deg, int nview, Grid g, Det d, double dsd,
-                                double dso, int geom, int ym, int xm, int hard) {
+                                double dso, int geom, int ym, int xm, int hard, int* __restrict__ order) {
     int j = blockIdx.x * blockDim.x + threadIdx.x;
     int view = blockIdx.y;
+    if (order && blockIdx.x == gridDim.x - 1) {
+        if (view == 0) order_blend_first(order, deg, nview, hard);
+        return;
+    }
     if (j > d.nu || view >= nview) return;
     double th = (double)deg[view];
     double sx, sy, ex, ey;
@@ -160,11 +218,7 @@ __global__ void dd_table_kernel(DDTabW t, const float* __restrict__ deg, int nvi
         t.cL[1][ic] = (float)((double)g.dx / fabs(sin(th - a)));
     }
     if (j == 0) {
-        double s, c;
-        sincos(th, &s, &c);
-        double r = (fabs(c) - fabs(s) + kDDMarginD) / (2 * kDDMarginD);
-        t.wx[view] = hard ? (fabsf(__cosf(deg[view])) > fabsf(__sinf(deg[view])) ? 1.f : 0.f)
-                          : (float)(r < 0 ? 0.0 : (r > 1 ? 1.0 : r));
+        t.wx[view] = view_weight(deg[view], hard);
         // fan source in line coordinates: edge j sits at sP + eB_j (t - sS) on
         // line t (counted from the anchor line)
         t.sP[0][view] = (float)sx;
@@ -1097,45 +1151,6 @@ __device__ unsigned int g_first_wait_polls = kWaitPolls;
 template <bool FAN, int NI>
 constexpr int fp_stream_min_blocks() { return NI <= 8 ? 3 : 2; }
 
-// The views in the order the streamed forward projector takes them: those of
-// the blend band (0 < wx < 1), which sweep both orientations and so take
-// about twice as long, first, then the others, each in their original order
-// (a stable partition).  The launch dispatches view groups in this order, so
-// its longest CTAs start in the first wave instead of trailing the last.
-// One CTA; ballots and per-warp counts give each view its position.
-__global__ void __launch_bounds__(1024) blend_first_kernel(int* __restrict__ order, const float* __restrict__ wx,
-                                                           int nview) {
-    __shared__ int s_cnt[32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    auto in_band = [&](int v) { return v < nview && wx[v] > 0.f && wx[v] < 1.f; };
-    int nband = 0;
-    for (int t0 = 0; t0 < nview; t0 += blockDim.x) nband += __syncthreads_count(in_band(t0 + threadIdx.x));
-    int placed_band = 0, placed_rest = 0;
-    for (int t0 = 0; t0 < nview; t0 += blockDim.x) {
-        const int v = t0 + threadIdx.x;
-        const bool in = v < nview, band = in_band(v);
-        const unsigned mb = __ballot_sync(0xffffffffu, band), mi = __ballot_sync(0xffffffffu, in);
-        const unsigned below = (1u << lane) - 1u;
-        if (lane == 0) s_cnt[warp] = __popc(mb) | (__popc(mi) << 16);
-        __syncthreads();
-        int band_before = __popc(mb & below), all_before = __popc(mi & below), tile_band = 0, tile_all = 0;
-        for (int w = 0; w < nw; ++w) {
-            const int c = s_cnt[w];
-            if (w < warp) {
-                band_before += c & 0xffff;
-                all_before += c >> 16;
-            }
-            tile_band += c & 0xffff;
-            tile_all += c >> 16;
-        }
-        if (in)
-            order[band ? placed_band + band_before : nband + placed_rest + (all_before - band_before)] = v;
-        placed_band += tile_band;
-        placed_rest += tile_all - tile_band;
-        __syncthreads();
-    }
-}
-
 template <bool FAN, int NI, typename Tout>
 __global__ void __launch_bounds__(256, (fp_stream_min_blocks<FAN, NI>())) dd2d_fp_stream_kernel(Tout* __restrict__ prj, const unsigned char* __restrict__ ltab0,
                                                              const unsigned char* __restrict__ ltab1, DDTab tab, Grid g,
@@ -1379,14 +1394,14 @@ int fp_stream_chunk(const ctp_geometry& g) {
 
 // hard != 0: the branchless tracer's per-view weights (main axis alone)
 int build_table(float* base, const float* deg, const ctp_geometry& g, int geom, cudaStream_t s, DDTab& tab,
-                int hard = 0) {
+                int hard = 0, int* order = nullptr) {
     DDTabW w;
     carve_table(base, g.nview, g.nu, w);
     int ym = (int)(g.ny / 2), xm = (int)(g.nx / 2);
     double dsd = geom == 0 ? g.dsd : 1000.0, dso = geom == 0 ? g.dso : 500.0;
-    dim3 grid((unsigned)((g.nu + 1 + 127) / 128), (unsigned)g.nview);
+    dim3 grid((unsigned)((g.nu + 1 + 127) / 128 + (order ? 1 : 0)), (unsigned)g.nview);
     dd_table_kernel<<<grid, 128, 0, s>>>(w, deg, (int)g.nview, make_grid(g), make_det(g), dsd, dso, geom, ym, xm,
-                                         hard);
+                                         hard, order);
     tab = as_read(w, ym, xm);
     return check_launch("dd_table_kernel");
 }
@@ -1495,7 +1510,10 @@ template <typename Tin, typename Tout>
 int launch_fp(void* prj, const void* img, const float* deg, const ctp_geometry& g, int geom, int type,
               unsigned flags, char* ws, size_t ws_bytes, cudaStream_t s) {
     DDTab tab;
-    int rc = build_table(reinterpret_cast<float*>(ws), deg, g, geom, s, tab, (type & CTP_TYPE_BRANCHLESS) ? 1 : 0);
+    // the views' order for the streamed path, made by the same launch
+    int* order = reinterpret_cast<int*>(ws + align_up(table_floats(g.nview, g.nu) * sizeof(float)));
+    int rc = build_table(reinterpret_cast<float*>(ws), deg, g, geom, s, tab, (type & CTP_TYPE_BRANCHLESS) ? 1 : 0,
+                         order);
     if (rc) return rc;
     Tin* imgT = reinterpret_cast<Tin*>(ws + fp_edge_table_bytes(g));
     const size_t slice_px = g.ny * g.nx;
@@ -1548,9 +1566,6 @@ int launch_fp(void* prj, const void* img, const float* deg, const ctp_geometry& 
         size_t shm = 2 * (size_t)rc_s * line_bytes((int)std::max(g.nx, g.ny));
         const bool fan = geom == 0;
         const int wpv = fan ? 8 / sv : 0;  // fan beams: warps per view (fp_item)
-        int* order = reinterpret_cast<int*>(ws + align_up(table_floats(g.nview, g.nu) * sizeof(float)));
-        blend_first_kernel<<<1, 1024, 0, s>>>(order, tab.wx, (int)g.nview);
-        if ((rc = check_launch("blend_first_kernel"))) return rc;
         for (int s0 = 0; s0 < nslices; s0 += chunk) {
             const int cs = std::min(chunk, nslices - s0);
             const Tin* from = cptr<Tin>(img) + (size_t)s0 * slice_px;
