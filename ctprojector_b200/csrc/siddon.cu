@@ -473,7 +473,7 @@ int siddon_fp(void* prj, const void* img, const float* dc, const float* du_, con
                                : launch_siddon_fp<long long>(prj, img, dc, du_, dv_, sr, rest, g, flags, s);
     };
     // upright views column by column, when the scratch can be had; the others ray by ray
-    if (columns_fp_applies(g)) {
+    if (columns_fp_applies(g, flags)) {
         Scratch scr;
         if (!scr.acquire(nullptr, 0, columns_fp_bytes(g, flags), s)) {
             ColumnsPlan plan;
@@ -497,7 +497,7 @@ int siddon_bp(void* img, const void* prj, const float* dc, const float* du_, con
         return small_volume(g) ? launch_siddon_bp<int>(img, prj, dc, du_, dv_, sr, rest, g, flags, s)
                                : launch_siddon_bp<long long>(img, prj, dc, du_, dv_, sr, rest, g, flags, s);
     };
-    if (columns_bp_applies(g)) {
+    if (columns_bp_applies(g, flags)) {
         Scratch scr;
         if (!scr.acquire(nullptr, 0, columns_bp_bytes(g), s)) {
             ColumnsPlan plan;

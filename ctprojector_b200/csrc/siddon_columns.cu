@@ -583,7 +583,8 @@ __device__ __forceinline__ bool bp_view(const UprightView& w, int tx0, int ty0, 
     return V.g0 < V.g1 && V.c1 > 0 && V.nrow > 0;
 }
 
-// Whether a view's window and rows fit the staged ones.
+// Whether a view's window and rows fit the staged ones (nrow <= nv + 1 <= rows +
+// 1 where the launch stages fewer rows than kBpRows).
 __device__ __forceinline__ bool bp_fits(const BpView& V) { return V.c1 <= kBpWin && V.nrow <= kBpRows + 1; }
 
 // Views that do not fit on some tile and z range (a coarse grid under a fine
@@ -632,8 +633,8 @@ template <bool ATOMIC>
 __global__ void __launch_bounds__(256, 2) columns_bp_kernel(float* __restrict__ img, const float* __restrict__ P,
                                                             const double2* __restrict__ inv,
                                                             const UprightView* __restrict__ views, int view0,
-                                                            int nviews, int vper, Grid g, Det d, int pitch, int zper,
-                                                            int zchunks) {
+                                                            int nviews, int vper, Grid g, Det d, int pitch, int rows,
+                                                            int zper, int zchunks) {
     extern __shared__ float4 s_raw[];
     float* s_P = reinterpret_cast<float*>(s_raw);     // [2][kBpStep][kBpRows + 1][kBpWin]
     float* s_split = s_P + kBpStageFloats;            // [kBpZ + 1][256] sums of the split rows, per plane and thread
@@ -698,7 +699,7 @@ __global__ void __launch_bounds__(256, 2) columns_bp_kernel(float* __restrict__ 
             const float* src = Pb + (size_t)V.vi * (d.nv + 1) * pitch + V.first + 4 * half;
             const int row = V.row, c1 = V.c1;
             if (4 * half < c1)
-                for (int r = 2 * (tid >> 5) + (lane >> 4); r <= kBpRows; r += 16)
+                for (int r = 2 * (tid >> 5) + (lane >> 4); r <= rows; r += 16)
                     cp_async16(dst + r * kBpWin, src + (size_t)min(row + r, d.nv) * pitch);
             const int c = tid - j * 64;  // (warps 0, 1 and 2, 3; rows: 4, 5 and 6, 7)
             if (c >= 0 && c < c1) s_line[buf][j][c] = line(V, c);
@@ -710,9 +711,10 @@ __global__ void __launch_bounds__(256, 2) columns_bp_kernel(float* __restrict__ 
 
     // Detector column c of the view V staged in buf, j against this thread's pixel.
     // A running sum is read at the column's base plus the bits of ceil(v) times
-    // the row's bytes; ceil is one directed rounding, and its clamps to [0,
-    // kBpRows] come with the saturating multiply-add before it (v scaled by a
-    // power of two, which rounds alike).
+    // the row's bytes; ceil is one directed rounding, and its clamps to [0, rows]
+    // come with the saturating multiply-add before it (v scaled by a power of
+    // two, which rounds alike).
+    const float frows = (float)rows, irows = 1.f / frows;
     auto column = [&](const BpView& V, int buf, int j, int c) {
         const float4 L = s_line[buf][j][c];
         const float* col = s_P + (buf * kBpStep + j) * kBpWindow + c;
@@ -728,12 +730,12 @@ __global__ void __launch_bounds__(256, 2) columns_bp_kernel(float* __restrict__ 
         const float zz0 = V.zz0, vc = V.vc, kbf = V.kbf, kvf = V.kvf;
         unsigned split = 0;  // planes 0 .. 31 that a row passes through inside the pixel
         bool split_top = false;
-        const float gA1 = gA * (1.f / kBpRows), gB1 = gB * (1.f / kBpRows), vc1 = vc * (1.f / kBpRows);
+        const float gA1 = gA * irows, gB1 = gB * irows, vc1 = vc * irows;
         const unsigned at = (unsigned)__cvta_generic_to_shared(col) - (unsigned)kMagicBits * (4u * kBpWin);
         auto plane = [&](int q) {
             const float zz = zz0 + (float)q;
-            const unsigned iA = __float_as_uint(__fmaf_ru(fma_sat(zz, gA1, vc1), (float)kBpRows, kMagic));
-            const unsigned iB = __float_as_uint(__fmaf_ru(fma_sat(zz, gB1, vc1), (float)kBpRows, kMagic));
+            const unsigned iA = __float_as_uint(__fmaf_ru(fma_sat(zz, gA1, vc1), frows, kMagic));
+            const unsigned iB = __float_as_uint(__fmaf_ru(fma_sat(zz, gB1, vc1), frows, kMagic));
             if (iA != iB) {
                 if (q < 32) split |= 1u << q;
                 else split_top = true;
@@ -760,8 +762,8 @@ __global__ void __launch_bounds__(256, 2) columns_bp_kernel(float* __restrict__ 
             if (split) split &= split - 1;
             else split_top = false;
             const float zz = zz0 + (float)q;
-            const int kA = __float_as_int(__fmaf_ru(fma_sat(zz, gA1, vc1), (float)kBpRows, kMagic)) - kMagicBits;
-            const int kB = __float_as_int(__fmaf_ru(fma_sat(zz, gB1, vc1), (float)kBpRows, kMagic)) - kMagicBits;
+            const int kA = __float_as_int(__fmaf_ru(fma_sat(zz, gA1, vc1), frows, kMagic)) - kMagicBits;
+            const int kB = __float_as_int(__fmaf_ru(fma_sat(zz, gB1, vc1), frows, kMagic)) - kMagicBits;
             // row k is at z = zs + alpha kappa: its part on A's side of the plane is
             // (z - zs - aA kappa) / ((aB - aA) kappa); the numerator cancels, so it is
             // taken from the row's z at the tile centre (row_z)
@@ -892,8 +894,20 @@ int setup_views(ColumnsPlan& plan, char* base, const float* dc, const float* du_
 
 }  // namespace
 
-bool columns_fp_applies(const ctp_geometry& g) {
-    return g.nv >= 8 && fp_item_elems(g) < (1ull << 31) && g.nview * g.nbatch <= 65535 &&
+// By size: the lanes that have a row (three quarters at least, of 32 rows or
+// more) and nearly two waves of blocks, below which the list's chain of loads is
+// exposed.  By rays and by columns: 42 x 172 x 176 voxels, 71 views of 274 x 47
+// cells (98%, 1278 blocks) 235 and 180 us; 33 x 187 x 201, 97 of 251 x 37 (77%)
+// 277 and 226; 24 x 388 x 379, 107 of 432 x 17 (53%) 422 and 449; 13 x 173 x 192,
+// 137 of 283 x 9 134 and 136.
+bool columns_fp_applies(const ctp_geometry& g, unsigned flags) {
+    if (g.nv < 8) return false;
+    int passes = 0;
+    const int rows = fp_rows(g, passes);
+    const size_t lanes = (size_t)passes * ((rows + 15) / 16) * 16;
+    const size_t blocks = (g.nu + 8 * kFpCols - 1) / (8 * kFpCols) * passes * g.nview * g.nbatch;
+    if (!(flags & CTP_FLAG_SIDDON_COLUMNS) && (g.nv < 32 || 4 * g.nv < 3 * lanes || blocks < 1200)) return false;
+    return fp_item_elems(g) < (1ull << 31) && g.nview * g.nbatch <= 65535 &&
            ((g.nz + 31) / 32) * g.nbatch <= 65535 && g.ny <= 65535;
 }
 
@@ -928,7 +942,20 @@ size_t bp_views(const ctp_geometry& g) {
 
 }  // namespace
 
-bool columns_bp_applies(const ctp_geometry& g) {
+// By size, from the two kernels' times (ms): a ray costs its crossings (0.58e9
+// cells of detector row times pixels per ms: 14.9 ms at 64 x 512 x 512 voxels
+// under 360 views of 736 x 64 cells, 0.34 at 33 x 187 x 201 under 97 of 251 x
+// 37), a crossing line 40 instructions a z range and 10 a plane whatever the
+// rows.  The factor and the 0.06 ms (nine launches) are where both take the same
+// time: 13 x 260 x 317 voxels, 284 views of 346 x 11 cells 585 us by rays, 659 by
+// columns; 42 x 106 x 110, 238 of 119 x 35 273 and 323; the other side 21 x 394 x
+// 384, 143 of 596 x 22 1113 and 870; 27 x 242 x 262, 148 of 294 x 25 (forward and
+// back) 951 and 754.
+bool columns_bp_applies(const ctp_geometry& g, unsigned flags) {
+    const double lines = (double)g.nview * g.nbatch * g.nu * std::max(g.nx, g.ny);
+    const double ray = lines * g.nv / 0.58e9;
+    const double column = lines * 1.27 * (40.0 * ((g.nz + kBpZ - 1) / kBpZ) + 10.0 * g.nz) / 2.14e10;
+    if (!(flags & CTP_FLAG_SIDDON_COLUMNS) && ray < 1.75 * column + 0.06) return false;
     return g.nz >= 4 && g.nv >= 2 && g.nbatch <= 65535 && g.nview <= 65535 && bp_view_bytes(g) <= kPrefixBytes &&
            g.nu < (1u << 28);
 }
@@ -990,9 +1017,12 @@ int columns_bp(ColumnsPlan& plan, char* scratch, float* img, const void* prj, co
         }
         const int vper = (n + parts - 1) / parts;
         const dim3 grid((unsigned)tiles, (unsigned)(zchunks * parts), (unsigned)g.nbatch);
+        int rows = 8;  // rows staged: a power of two (see column), nv or more up to kBpRows
+        while (rows < kBpRows && rows < (int)g.nv) rows *= 2;
         auto k = parts > 1 ? columns_bp_kernel<true> : columns_bp_kernel<false>;
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k<<<grid, 256, smem, s>>>(img, P, inv, plan.views, (int)v0, n, vper, gr, dt, (int)bp_pitch(g), zper, zchunks);
+        k<<<grid, 256, smem, s>>>(img, P, inv, plan.views, (int)v0, n, vper, gr, dt, (int)bp_pitch(g), rows, zper,
+                                  zchunks);
         if ((rc = check_launch("columns_bp_kernel"))) return rc;
     }
     return CTP_OK;

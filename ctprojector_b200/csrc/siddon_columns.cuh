@@ -25,9 +25,9 @@ struct ColumnsPlan {
 };
 
 // Whether the sizes suit the column kernels, and the scratch they take.
-bool columns_fp_applies(const ctp_geometry& g);
+bool columns_fp_applies(const ctp_geometry& g, unsigned flags);
 size_t columns_fp_bytes(const ctp_geometry& g, unsigned flags);
-bool columns_bp_applies(const ctp_geometry& g);
+bool columns_bp_applies(const ctp_geometry& g, unsigned flags);
 size_t columns_bp_bytes(const ctp_geometry& g);
 
 // The upright views of a call; the caller runs the ray-driven kernel on

@@ -67,6 +67,8 @@ extern "C" {
 #define CTP_FLAG_FILTER_EXACT 0x100 /* ramp filter: FP64 windowed kernel, smooth FFT size
                                        (default: the reference's FP32 construction) */
 #define CTP_FLAG_SUBTRACT 0x400 /* ctp_dequantize_u16: subtract the values from the output */
+#define CTP_FLAG_SIDDON_COLUMNS 0x800 /* Siddon pair: upright views column by column at any size the kernels
+                                        take (by default where the size makes that faster) */
 
 /* typeProjector bits of the DD 2D entries, as in the reference
  * (distanceDriven2D.cu:12-25): bit0 FBP weighting, bit1 branchless,

@@ -17,10 +17,17 @@ torch = pytest.importorskip("torch")
 TOL = 4e-6
 
 
-@pytest.fixture(scope="module", autouse=True)
-def _cuda():
+SIDDON_COLUMNS = 0x800  # CTP_FLAG_SIDDON_COLUMNS: the column kernels at these sizes too
+
+
+@pytest.fixture(autouse=True)
+def _columns(monkeypatch):
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
+    from ctprojector_b200.projector import _device
+
+    flags = _device._io_flags
+    monkeypatch.setattr(_device, "_io_flags", lambda a, b: flags(a, b) | SIDDON_COLUMNS)
 
 
 def scan(nx, ny, nz, nu, nv, nview=13, pixel=3.0, dz=2.0, cell=None, row=None, **kw):
