@@ -363,9 +363,18 @@ int get_ref_plan(int L, int nu, int batch, RefPlan** out) {
     return CTP_OK;
 }
 
+// Padded rows are transformed `batch` at a time.  cuFFT takes real data on 8-byte
+// boundaries only, so where a batch is an odd number of floats (an odd number of
+// rows: L is odd), the next one starts one float later.
+size_t pad_batch_floats(int L, int batch) { return ((size_t)L * batch + 1) & ~(size_t)1; }
+size_t pad_floats(int L, int batch, size_t rows) { return (rows + batch - 1) / batch * pad_batch_floats(L, batch); }
+__device__ __forceinline__ size_t pad_row(size_t r, int L, int batch) {
+    return r * L + (L & batch & 1 ? r / batch : 0);
+}
+
 // CopyPrjToPad + Multiply2D (fbpMath.cu:59-72, cudaMath.cu:28-49): one pass over all rows.
 __global__ void ref_pad_kernel(float* __restrict__ pad, const float* __restrict__ prj, const float* __restrict__ w,
-                               int nu, int L, size_t rows) {
+                               int nu, int L, int batch, size_t rows) {
     size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (i >= rows * L) return;
     size_t r = i / L;
@@ -375,7 +384,7 @@ __global__ void ref_pad_kernel(float* __restrict__ pad, const float* __restrict_
         v = prj[r * nu + n];
         if (w) v = v * w[n];
     }
-    pad[i] = v;
+    pad[pad_row(r, L, batch) + n] = v;
 }
 
 // ComplexMultiply2D (fbpMath.cu:12-33) against the kernel replicated over rows.
@@ -392,20 +401,21 @@ __global__ void ref_cmul_kernel(cufftComplex* __restrict__ f, const cufftComplex
 }
 
 // Scale2D + CopyPadToPrj (cudaMath.cu:76-97, fbpMath.cu:74-87).
-__global__ void ref_crop_kernel(float* __restrict__ out, const float* __restrict__ pad, int nu, int L, size_t rows,
-                                float scale) {
+__global__ void ref_crop_kernel(float* __restrict__ out, const float* __restrict__ pad, int nu, int L, int batch,
+                                size_t rows, float scale) {
     size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (i >= rows * nu) return;
     size_t r = i / nu;
     int n = (int)(i - r * nu);
-    out[i] = pad[r * L + nu - 1 + n] * scale;
+    out[i] = pad[pad_row(r, L, batch) + nu - 1 + n] * scale;
 }
 
 size_t ref_workspace(const ctp_geometry& g) {
     size_t nu = g.nu, L = 2 * nu - 1, rows = g.nbatch * g.nview * g.nv;
     RefPlan* p = nullptr;
     if (get_ref_plan((int)L, (int)nu, (int)g.nview, &p)) return 0;
-    return align_up(rows * L * sizeof(float)) + align_up(rows * nu * sizeof(cufftComplex)) + align_up(p->work);
+    return align_up(pad_floats((int)L, (int)g.nview, rows) * sizeof(float)) +
+           align_up(rows * nu * sizeof(cufftComplex)) + align_up(p->work);
 }
 
 int ramp_filter_reference(float* fprj, const float* prj, const ctp_geometry& g, int geom, int filter,
@@ -419,7 +429,7 @@ int ramp_filter_reference(float* fprj, const float* prj, const ctp_geometry& g, 
     RefPlan* plan = nullptr;
     if ((rc = get_ref_plan(L, nu, nview, &plan))) return rc;
     Scratch scr;
-    size_t pad_b = align_up(rows * L * sizeof(float)), frq_b = align_up(rows * nu * sizeof(cufftComplex));
+    size_t pad_b = align_up(pad_floats(L, nview, rows) * sizeof(float)), frq_b = align_up(rows * nu * sizeof(cufftComplex));
     if ((rc = scr.acquire(workspace, workspace_bytes, pad_b + frq_b + align_up(plan->work), s))) return rc;
     float* pad = reinterpret_cast<float*>(scr.base());
     cufftComplex* frq = reinterpret_cast<cufftComplex*>(scr.base() + pad_b);
@@ -428,7 +438,7 @@ int ramp_filter_reference(float* fprj, const float* prj, const ctp_geometry& g, 
     // fbpParallel.cu:59, fbp.cu:103 (float arithmetic)
     float scale = fan ? PIf / g.nview * g.du / g.dso / L : PIf / g.nview * g.du / L;
     size_t np = rows * L;
-    ref_pad_kernel<<<(unsigned)((np + 255) / 256), 256, 0, s>>>(pad, prj, fan ? rf.weight : nullptr, nu, L, rows);
+    ref_pad_kernel<<<(unsigned)((np + 255) / 256), 256, 0, s>>>(pad, prj, fan ? rf.weight : nullptr, nu, L, nview, rows);
     if ((rc = check_launch("ref_pad_kernel"))) return rc;
     {
         std::lock_guard<std::mutex> lk(plan->mu);
@@ -436,18 +446,19 @@ int ramp_filter_reference(float* fprj, const float* prj, const ctp_geometry& g, 
         cufftSetStream(plan->inv, s);
         cufftSetWorkArea(plan->fwd, work);
         cufftSetWorkArea(plan->inv, work);
+        const size_t batch_floats = pad_batch_floats(L, nview);
         for (size_t r0 = 0; r0 < rows; r0 += nview)
-            if (cufftExecR2C(plan->fwd, pad + r0 * L, frq + r0 * nu) != CUFFT_SUCCESS)
+            if (cufftExecR2C(plan->fwd, pad + r0 / nview * batch_floats, frq + r0 * nu) != CUFFT_SUCCESS)
                 return set_error(CTP_ERR_CUFFT, "cufftExecR2C failed");
         size_t nf = rows * nu;
         ref_cmul_kernel<<<(unsigned)((nf + 255) / 256), 256, 0, s>>>(frq, rf.spec, nu, rows);
         if ((rc = check_launch("ref_cmul_kernel"))) return rc;
         for (size_t r0 = 0; r0 < rows; r0 += nview)
-            if (cufftExecC2R(plan->inv, frq + r0 * nu, pad + r0 * L) != CUFFT_SUCCESS)
+            if (cufftExecC2R(plan->inv, frq + r0 * nu, pad + r0 / nview * batch_floats) != CUFFT_SUCCESS)
                 return set_error(CTP_ERR_CUFFT, "cufftExecC2R failed");
     }
     size_t no = rows * nu;
-    ref_crop_kernel<<<(unsigned)((no + 255) / 256), 256, 0, s>>>(fprj, pad, nu, L, rows, scale);
+    ref_crop_kernel<<<(unsigned)((no + 255) / 256), 256, 0, s>>>(fprj, pad, nu, L, nview, rows, scale);
     return check_launch("ref_crop_kernel");
 }
 
@@ -970,7 +981,7 @@ __global__ void tomo_crop_kernel(float* __restrict__ out, const float* __restric
     if (i >= rows * nu) return;
     size_t r = i / nu;
     int n = (int)(i - r * nu);
-    out[i] = pad[r * L + nu - 1 + n] * scale[(r / nv) % nview];
+    out[i] = pad[pad_row(r, L, nv) + nu - 1 + n] * scale[(r / nv) % nview];
 }
 
 }  // namespace
@@ -979,7 +990,8 @@ size_t tomo_filter_workspace(const ctp_geometry& g) {
     size_t nu = g.nu, L = 2 * nu - 1, rows = g.nbatch * g.nview * g.nv;
     RefPlan* p = nullptr;
     if (nu == 0 || g.nv == 0 || get_ref_plan((int)L, (int)nu, (int)g.nv, &p)) return 0;
-    return align_up(rows * L * sizeof(float)) + align_up(rows * nu * sizeof(cufftComplex)) + align_up(p->work) +
+    return align_up(pad_floats((int)L, (int)g.nv, rows) * sizeof(float)) +
+           align_up(rows * nu * sizeof(cufftComplex)) + align_up(p->work) +
            align_up(g.nview * nu * sizeof(cufftComplex)) + align_up(g.nview * sizeof(float));
 }
 
@@ -1011,7 +1023,7 @@ int tomo_filter(float* fprj, const float* prj, const float* det_center, const fl
     int rc = get_ref_plan(L, nu, nv, &plan);
     if (rc) return rc;
     Scratch scr;
-    size_t pad_b = align_up(rows * L * sizeof(float)), frq_b = align_up(rows * nu * sizeof(cufftComplex));
+    size_t pad_b = align_up(pad_floats(L, nv, rows) * sizeof(float)), frq_b = align_up(rows * nu * sizeof(cufftComplex));
     size_t work_b = align_up(plan->work), spec_b = align_up(g.nview * nu * sizeof(cufftComplex));
     if ((rc = scr.acquire(workspace, workspace_bytes, pad_b + frq_b + work_b + spec_b + align_up(g.nview * sizeof(float)),
                           s)))
@@ -1032,7 +1044,7 @@ int tomo_filter(float* fprj, const float* prj, const float* det_center, const fl
     e = cudaMemcpyAsync(dscale, scale.data(), sizeof(float) * nview, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return set_error((int)e, "tomo filter scales: %s", cudaGetErrorString(e));
-    ref_pad_kernel<<<(unsigned)((rows * L + 255) / 256), 256, 0, s>>>(pad, prj, nullptr, nu, L, rows);
+    ref_pad_kernel<<<(unsigned)((rows * L + 255) / 256), 256, 0, s>>>(pad, prj, nullptr, nu, L, nv, rows);
     if ((rc = check_launch("ref_pad_kernel"))) return rc;
     {
         std::lock_guard<std::mutex> lk(plan->mu);
@@ -1040,14 +1052,15 @@ int tomo_filter(float* fprj, const float* prj, const float* det_center, const fl
         cufftSetStream(plan->inv, s);
         cufftSetWorkArea(plan->fwd, work);
         cufftSetWorkArea(plan->inv, work);
+        const size_t batch_floats = pad_batch_floats(L, nv);
         for (size_t r0 = 0; r0 < rows; r0 += nv)
-            if (cufftExecR2C(plan->fwd, pad + r0 * L, frq + r0 * nu) != CUFFT_SUCCESS)
+            if (cufftExecR2C(plan->fwd, pad + r0 / nv * batch_floats, frq + r0 * nu) != CUFFT_SUCCESS)
                 return set_error(CTP_ERR_CUFFT, "cufftExecR2C failed");
         tomo_cmul_kernel<<<(unsigned)((rows * nu + 255) / 256), 256, 0, s>>>(frq, spec, nu, nv,
                                                                            first_only ? 1 : nview, rows);
         if ((rc = check_launch("tomo_cmul_kernel"))) return rc;
         for (size_t r0 = 0; r0 < rows; r0 += nv)
-            if (cufftExecC2R(plan->inv, frq + r0 * nu, pad + r0 * L) != CUFFT_SUCCESS)
+            if (cufftExecC2R(plan->inv, frq + r0 * nu, pad + r0 / nv * batch_floats) != CUFFT_SUCCESS)
                 return set_error(CTP_ERR_CUFFT, "cufftExecC2R failed");
     }
     tomo_crop_kernel<<<(unsigned)((rows * nu + 255) / 256), 256, 0, s>>>(fprj, pad, dscale, nu, L, nv, nview, rows);

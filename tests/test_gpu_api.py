@@ -227,3 +227,33 @@ def test_nnz_matches_oracle(oracle):
     a = [inp[k] for k in ("det_center", "det_u", "det_v", "src")]
     n = D.siddon_nnz(p, *[dev(v) for v in a], image_shape=inp["img"].shape[1:])
     assert abs(n - oracle.siddon_nnz(p, *a, shape=inp["img"].shape[1:])) <= 1e-4 * n
+
+
+@pytest.mark.parametrize("module", ["fan_equiangular", "parallel"])
+@pytest.mark.parametrize("nview,nu", [(7, 397), (8, 30), (5, 21)])
+def test_default_filter_of_a_batch_equals_its_items(module, nview, nu):
+    """Odd numbers of views of odd padded rows: items that start off an 8-byte boundary."""
+    import importlib
+
+    from cases import Proj
+
+    M = importlib.import_module("ctprojector_b200.projector.cupy." + module)
+    p = Proj(nx=32, ny=32, nu=nu, du=1.0, nview=nview)
+    prj = dev(np.random.default_rng(nu).uniform(0, 1, (3, nview, 1, nu)))
+    whole = host(M.ramp_filter(p, prj, "hann"))
+    for b in range(3):
+        np.testing.assert_array_equal(whole[b:b + 1], host(M.ramp_filter(p, prj[b:b + 1].contiguous(), "hann")))
+
+
+def test_tomo_filter_of_odd_rows_equals_its_views():
+    from cases import Proj
+
+    from ctprojector_b200 import synthetic as S
+    from ctprojector_b200.projector.cupy import tomo
+
+    p = Proj(nx=32, ny=32, nz=4, dx=0.4, dy=0.4, nu=37, nv=5, du=0.3, dv=0.3, nview=3)
+    dc, sr = (dev(a) for a in S.tomo_geometry(3, 40.0, 500.0, -20.0))
+    prj = dev(np.random.default_rng(1).uniform(0, 1, (2, 3, 5, 37)))
+    whole = host(tomo.filter_fbp(p, prj, dc, sr))
+    for b in range(2):
+        np.testing.assert_array_equal(whole[b:b + 1], host(tomo.filter_fbp(p, prj[b:b + 1].contiguous(), dc, sr)))
