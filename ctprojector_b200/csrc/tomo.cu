@@ -72,6 +72,23 @@ __device__ __forceinline__ Taps<K> taps(double lo, double hi, float inv, int n) 
     return t;
 }
 
+// A footprint that misses the array was clamped to cells of its border: they
+// are left unread (0 x infinity is not 0).  Along a row of a table the mark
+// kMissed on the first cell sends the lookup past the sums, to zeros.
+constexpr int kMissed = 0x40000000;
+template <int K>
+__device__ __forceinline__ bool missed(const Taps<K>& t) {
+    bool m = true;
+#pragma unroll
+    for (int k = 0; k < K; ++k) m = m && t.w[k] == 0.f;
+    return m;
+}
+template <int K>
+__device__ __forceinline__ float row_index(const Taps<K>& t) {
+    return __int_as_float(missed(t) ? t.i | kMissed : t.i);
+}
+__device__ __forceinline__ int first_row(float index) { return __float_as_int(index) & ~kMissed; }
+
 // A view's rays in image coordinates: source (sx, sy, sz), and the cell edges'
 // position on plane z: sx + r (z - sz).
 struct TomoRays {
@@ -126,7 +143,8 @@ __global__ void __launch_bounds__(kTomoThreads, 6) tomo_fp_kernel(float* __restr
                                                                   const float* __restrict__ dc,
                                                                   const float* __restrict__ sr, int nview, Grid g, Det d) {
     __shared__ float4 s_row[kTomoStep][VT];          // y weights of a cell row, its first image row
-    __shared__ float s_sum[VT + 4][kTomoThreads];    // each thread its own column: rows summed over x, then results
+    // each thread its own column: up to VT + 2 rows summed over x and two of zeros, then results
+    __shared__ float s_sum[VT + 4][kTomoThreads];
     const int tid = threadIdx.x;
     const int iu = blockIdx.x * kTomoThreads + tid;
     const int v0 = blockIdx.y * VT;
@@ -145,6 +163,7 @@ __global__ void __launch_bounds__(kTomoThreads, 6) tomo_fp_kernel(float* __restr
         float acc[VT];
 #pragma unroll
         for (int q = 0; q < VT; ++q) acc[q] = 0.f;
+        s_sum[VT + 2][tid] = s_sum[VT + 3][tid] = 0.f;
         for (int z0 = 0; z0 < g.nz; z0 += kTomoStep) {
             const int nz = min(kTomoStep, g.nz - z0);
             __syncthreads();
@@ -155,17 +174,18 @@ __global__ void __launch_bounds__(kTomoThreads, 6) tomo_fp_kernel(float* __restr
                 row_slopes(min(v0 + q, d.nv - 1), r1, r2);
                 const double dz = z0 + z - R.sz;
                 const Taps<2> t = taps<2>(R.sy + r1 * dz, R.sy + r2 * dz, (float)(1.0 / ((r2 - r1) * dz)), g.ny);
-                s_row[z][q] = make_float4(t.w[0], t.w[1], __int_as_float(t.i), 0.f);
+                s_row[z][q] = make_float4(t.w[0], t.w[1], row_index(t), 0.f);
             }
             __syncthreads();
 #pragma unroll 1
             for (int z = 0; z < nz; ++z) {
                 const double dz = z0 + z - R.sz;
                 const Taps<2> t = taps<2>(R.sx + rx1 * dz, R.sx + rx2 * dz, __fdividef(1.f, (float)((rx2 - rx1) * dz)), g.nx);
+                if (missed(t)) continue;
                 const int right = t.i + 1 < g.nx ? 1 : 0;
                 // image rows of the first and last cell (rows advance by at most one per cell)
-                const int ra = __float_as_int(s_row[z][0].z), rb = __float_as_int(s_row[z][VT - 1].z);
-                const int y0 = min(ra, rb), n = min(max(ra, rb) + 1 - y0, VT + 2);
+                const int ra = first_row(s_row[z][0].z), rb = first_row(s_row[z][VT - 1].z);
+                const int y0 = min(ra, rb), n = min(max(ra, rb) + 1 - y0, VT + 1);
                 const float* col = vol + ((size_t)(z0 + z) * g.ny + y0) * g.nx + t.i;
                 const int last = g.ny - 1 - y0;
 #pragma unroll 8
@@ -237,10 +257,10 @@ template <int YT>
 __global__ void __launch_bounds__(kTomoThreads, 5) tomo_bp_kernel(float* __restrict__ img, const float* __restrict__ wprj,
                                                                   const float* __restrict__ dc,
                                                                   const float* __restrict__ sr, int nview, Grid g, Det d) {
-    constexpr int kRows = 2 * YT + 4;                 // detector rows under YT voxels of at most 2 rows
+    constexpr int kRows = 2 * YT + 2;                 // detector rows under YT voxels of at most 2 rows
     __shared__ float4 s_row[kTomoStep][YT];           // v weights of a voxel row, its first detector row
     __shared__ double s_u[kTomoStep][2];              // u = s_u[0] + s_u[1] x
-    __shared__ float s_sum[kRows][kTomoThreads];      // each thread its own column: rows summed over u
+    __shared__ float s_sum[kRows + 3][kTomoThreads];  // each thread its own column: rows summed over u, three of zeros
     const int tid = threadIdx.x;
     const int ix = blockIdx.x * kTomoThreads + tid;
     const int y0 = blockIdx.y * YT;
@@ -251,6 +271,7 @@ __global__ void __launch_bounds__(kTomoThreads, 5) tomo_bp_kernel(float* __restr
     float acc[YT];
 #pragma unroll
     for (int q = 0; q < YT; ++q) acc[q] = 0.f;
+    s_sum[kRows][tid] = s_sum[kRows + 1][tid] = s_sum[kRows + 2][tid] = 0.f;
     // detector coordinate of the position p along one axis: lo + slope p
     auto mapping = [&](double S, double C, double cell, double off, int n, double r, double& c0, double& c1) {
         c1 = r / cell;
@@ -272,7 +293,7 @@ __global__ void __launch_bounds__(kTomoThreads, 5) tomo_bp_kernel(float* __restr
             mapping(sr[view * 3 + 1], dc[view * 3 + 1], d.dv, d.off_v, d.nv, r, c0, c1);
             const double y = voxel_y(q);
             const Taps<3> t = taps<3>(fma(c1, y - hy, c0), fma(c1, y + hy, c0), (float)(1.0 / (c1 * g.dy)), d.nv);
-            s_row[w][q] = make_float4(t.w[0], t.w[1], t.w[2], __int_as_float(t.i));
+            s_row[w][q] = make_float4(t.w[0], t.w[1], t.w[2], row_index(t));
             if (q == 0) mapping(sr[view * 3], dc[view * 3], d.du, d.off_u, d.nu, r, s_u[w][0], s_u[w][1]);
         }
         __syncthreads();
@@ -285,9 +306,10 @@ __global__ void __launch_bounds__(kTomoThreads, 5) tomo_bp_kernel(float* __restr
             const double wu = fabs(c1 * g.dx), wv = fabs(c1 * d.du / d.dv * g.dy);
             if (wu <= 2.0 && wv <= 2.0) {
                 const Taps<3> t = taps<3>(u1, u2, __fdividef(1.f, (float)(c1 * g.dx)), d.nu);
+                if (missed(t)) continue;
                 const int i1 = min(1, d.nu - 1 - t.i), i2 = min(2, d.nu - 1 - t.i);
                 // detector rows of the first and last voxel (rows advance by at most two per voxel)
-                const int ra = __float_as_int(s_row[w][0].w), rb = __float_as_int(s_row[w][YT - 1].w);
+                const int ra = first_row(s_row[w][0].w), rb = first_row(s_row[w][YT - 1].w);
                 const int v0 = min(ra, rb), n = min(max(ra, rb) + 3 - v0, kRows), last = d.nv - 1 - v0;
                 const float* col = pv + (size_t)v0 * d.nu + t.i;
 #pragma unroll 6
@@ -298,7 +320,7 @@ __global__ void __launch_bounds__(kTomoThreads, 5) tomo_bp_kernel(float* __restr
 #pragma unroll
                 for (int k = 0; k < YT; ++k) {
                     const float4 e = s_row[w][k];
-                    const int r = min(__float_as_int(e.w) - v0, kRows - 3);
+                    const int r = min(__float_as_int(e.w) - v0, kRows);
                     acc[k] = fmaf(e.x, s_sum[r][tid], fmaf(e.y, s_sum[r + 1][tid], fmaf(e.z, s_sum[r + 2][tid], acc[k])));
                 }
             } else {

@@ -47,3 +47,49 @@ def test_tomo_rows(nx, ny, nz, nu, nv, cell, oracle):
     tol = TOL if cell <= 0.4 else 182 / 0.4 * 2.0**-23
     assert rel_l2(fp, oracle.tomo_fp(p, img, dc, sr)) <= tol
     assert rel_l2(bp, oracle.tomo_bp(p, prj, dc, sr)) <= tol
+
+
+def scan(nx, ny, nz, nu, nv, cell, nview, **kw):
+    from cases import Proj
+
+    from ctprojector_b200 import synthetic as S
+
+    p = Proj(nx=nx, ny=ny, nz=nz, dx=0.4, dy=0.4, dz=1.0, nu=nu, nv=nv, du=cell, dv=cell, nview=nview, **kw)
+    dc, sr = S.tomo_geometry(nview, 40.0, 500.0, -(nz / 2 + 15.0))
+    return p, dc, sr
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_tomo_values_off_the_footprint_do_not_matter(bad, oracle):
+    """Cells and pixels that a footprint does not reach, though it was clamped
+    to the border they lie on, leave its result alone."""
+    p, dc, sr = scan(48, 40, 9, 100, 90, 0.3, 11)
+    rng = np.random.default_rng(2)
+    img = rng.uniform(0, 1, (1, 9, 40, 48)).astype(np.float32)
+    mark = np.zeros_like(img)
+    for z, y, x in ((4, 0, 20), (3, 39, 11), (6, 17, 0), (2, 25, 47), (5, 0, 0)):
+        img[0, z, y, x] = bad
+        mark[0, z, max(y - 1, 0):y + 2, max(x - 1, 0):x + 2] = 1
+    away = oracle.tomo_fp(p, mark, dc, sr) == 0
+    ref = oracle.tomo_fp(p, np.where(np.isfinite(img), img, 0).astype(np.float32), dc, sr)
+    out = tomo_call("distance_driven_fp", p, img, dc, sr)
+    assert away.any() and np.isfinite(out[away]).all()
+    assert rel_l2(out[away], ref[away]) <= TOL
+
+    p, dc, sr = scan(96, 80, 9, 40, 30, 0.3, 11)  # voxels past the detector's borders
+    prj = rng.uniform(0, 1, (1, 11, 30, 40)).astype(np.float32)
+    mark = np.zeros_like(prj)
+    for view, v, u in ((0, 0, 20), (3, 29, 11), (6, 17, 0), (9, 25, 39), (10, 29, 39)):
+        prj[0, view, v, u] = bad
+        mark[0, view, max(v - 2, 0):v + 3, max(u - 2, 0):u + 3] = 1
+    away = oracle.tomo_bp(p, mark, dc, sr) == 0
+    ref = oracle.tomo_bp(p, np.where(np.isfinite(prj), prj, 0).astype(np.float32), dc, sr)
+    out = tomo_call("distance_driven_bp", p, prj, dc, sr)
+    assert away.any() and np.isfinite(out[away]).all()
+    assert rel_l2(out[away], ref[away]) <= TOL
+
+
+def tomo_call(name, p, x, dc, sr):
+    from ctprojector_b200.projector.cupy import tomo
+
+    return getattr(tomo, name)(p, dev(x), dev(dc), dev(sr)).cpu().numpy()
