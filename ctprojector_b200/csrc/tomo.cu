@@ -224,19 +224,21 @@ __global__ void __launch_bounds__(kTomoThreads, 6) tomo_fp_kernel(float* __restr
     }
 }
 
-// Length-weighted projections; the sum of squares in FP64, its root in FP32.
+// Length-weighted projections, one cell per thread of a one-dimensional grid
+// (views x batch items may exceed a grid's third dimension).
 __global__ void tomo_preweight_kernel(float* __restrict__ out, const float* __restrict__ prj,
                                       const float* __restrict__ dc, const float* __restrict__ sr, int nview, Det d,
-                                      float dz) {
-    const int iu = blockIdx.x * blockDim.x + threadIdx.x;
-    const int iv = blockIdx.y, view = blockIdx.z % nview;
+                                      float dz, unsigned blocks_u) {
+    const unsigned row = blockIdx.x / blocks_u;  // of all views and batch items
+    const int iu = (int)(blockIdx.x - row * blocks_u) * blockDim.x + threadIdx.x;
     if (iu >= d.nu) return;
+    const int iv = (int)(row % d.nv), view = (int)(row / d.nv % nview);
     const double u = ((double)iu - d.off_u - (d.nu - 1) / 2.0) * d.du + dc[view * 3] - sr[view * 3];
     const double v = ((double)iv - d.off_v - (d.nv - 1) / 2.0) * d.dv + dc[view * 3 + 1] - sr[view * 3 + 1];
     const double h = (double)dc[view * 3 + 2] - sr[view * 3 + 2];
     // L / |h| * dz
     const float q = (float)((u * u + v * v + h * h) * ((double)dz * dz / (h * h)));
-    const size_t i = ((size_t)blockIdx.z * d.nv + iv) * d.nu + iu;
+    const size_t i = (size_t)row * d.nu + iu;
     out[i] = prj[i] * sqrtf(q);
 }
 
@@ -523,8 +525,9 @@ int tomo_bp(float* img, const float* prj, const float* dc, const float* sr, cons
     int rc = scr.acquire(workspace, workspace_bytes, tomo_bp_workspace(g), s);
     if (rc) return rc;
     float* wprj = reinterpret_cast<float*>(scr.base());
-    tomo_preweight_kernel<<<dim3((unsigned)((g.nu + 127) / 128), (unsigned)g.nv, (unsigned)(g.nview * g.nbatch)), 128, 0,
-                            s>>>(wprj, prj, dc, sr, (int)g.nview, make_det(g), g.dz);
+    const size_t blocks_u = (g.nu + 127) / 128;
+    tomo_preweight_kernel<<<(unsigned)(blocks_u * g.nv * g.nview * g.nbatch), 128, 0, s>>>(
+        wprj, prj, dc, sr, (int)g.nview, make_det(g), g.dz, (unsigned)blocks_u);
     if ((rc = check_launch("tomo_preweight_kernel"))) return rc;
     (void)flags;
     if (!shared_rows(g)) {

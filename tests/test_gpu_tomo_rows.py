@@ -93,3 +93,12 @@ def tomo_call(name, p, x, dc, sr):
     from ctprojector_b200.projector.cupy import tomo
 
     return getattr(tomo, name)(p, dev(x), dev(dc), dev(sr)).cpu().numpy()
+
+
+def test_tomo_bp_more_views_than_a_grid_dimension(oracle):
+    """Views times batch items past 65535."""
+    nview = 33000
+    p, dc, sr = scan(5, 4, 1, 6, 5, 0.3, nview)
+    prj = np.random.default_rng(0).uniform(0, 1, (2, nview, 5, 6)).astype(np.float32)
+    # 33000 terms in one FP32 sum: sqrt(33000 / 3) 2^-24 = 6e-6
+    assert rel_l2(tomo_call("distance_driven_bp", p, prj, dc, sr), oracle.tomo_bp(p, prj, dc, sr)) <= 1.2e-5
