@@ -236,10 +236,8 @@ __global__ void tomo_preweight_kernel(float* __restrict__ out, const float* __re
     const double u = ((double)iu - d.off_u - (d.nu - 1) / 2.0) * d.du + dc[view * 3] - sr[view * 3];
     const double v = ((double)iv - d.off_v - (d.nv - 1) / 2.0) * d.dv + dc[view * 3 + 1] - sr[view * 3 + 1];
     const double h = (double)dc[view * 3 + 2] - sr[view * 3 + 2];
-    // L / |h| * dz
-    const float q = (float)((u * u + v * v + h * h) * ((double)dz * dz / (h * h)));
     const size_t i = (size_t)row * d.nu + iu;
-    out[i] = prj[i] * sqrtf(q);
+    out[i] = prj[i] * (float)(dz / fabs(h) * sqrt(u * u + v * v + h * h));
 }
 
 // Normalised integral of a view over one voxel's wide footprint (more than 3 x 3 cells).

@@ -102,3 +102,19 @@ def test_tomo_bp_more_views_than_a_grid_dimension(oracle):
     prj = np.random.default_rng(0).uniform(0, 1, (2, nview, 5, 6)).astype(np.float32)
     # 33000 terms in one FP32 sum: sqrt(33000 / 3) 2^-24 = 6e-6
     assert rel_l2(tomo_call("distance_driven_bp", p, prj, dc, sr), oracle.tomo_bp(p, prj, dc, sr)) <= 1.2e-5
+
+
+def test_tomo_ray_length_weight_is_rounded_once():
+    """A panel in the plane of the voxels, one voxel per cell: the voxels of a
+    projection of ones are the cells' weights, FP64 values rounded to FP32."""
+    from cases import Proj
+
+    n, m = 200, 150
+    p = Proj(nx=n, ny=m, nz=1, dx=0.5, dy=0.5, dz=1.0, nu=n, nv=m, du=0.5, dv=0.5, nview=1, off_u=0.5, off_v=0.5)
+    sr = np.array([[13.3, -7.1, 613.7]], np.float32)
+    out = tomo_call("distance_driven_bp", p, np.ones((1, 1, m, n)), np.zeros((1, 3)), sr)[0, 0]
+    s = sr[0].astype(np.float64)
+    u = (np.arange(n) - 0.5 - (n - 1) / 2) * 0.5 - s[0]
+    v = (np.arange(m) - 0.5 - (m - 1) / 2) * 0.5 - s[1]
+    ref = (1 / abs(s[2]) * np.sqrt(u * u + v[:, None] ** 2 + s[2] ** 2)).astype(np.float32)
+    assert (out != ref).mean() < 1e-3
