@@ -34,8 +34,6 @@
 
 #include <algorithm>
 #include <atomic>
-#include <cfloat>
-#include <cmath>
 #include <climits>
 #include <type_traits>
 
@@ -238,45 +236,19 @@ __global__ void dd_table_kernel(DDTabW t, const float* __restrict__ deg, int nvi
 // trigonometry.
 __device__ __forceinline__ bool ref_y_main(float deg) { return fabsf(__cosf(deg)) > fabsf(__sinf(deg)); }
 
-// [nslice][ny][nx] -> [nslice][nx][ny].  stats (may be null): per 32 x 32 tile
-// the largest magnitude (infinite when a value is not finite) and the sum of
-// magnitudes, stats[slice][tile].
+// [nslice][ny][nx] -> [nslice][nx][ny]
 template <typename T>
-__global__ void transpose_kernel(T* __restrict__ out, const T* __restrict__ in, int nx, int ny,
-                                 float2* __restrict__ stats) {
+__global__ void transpose_kernel(T* __restrict__ out, const T* __restrict__ in, int nx, int ny) {
     __shared__ T tile[32][33];
-    __shared__ float2 s_red[8];
     size_t slice = blockIdx.z;
     const T* src = in + slice * (size_t)nx * ny;
     T* dst = out + slice * (size_t)nx * ny;
     int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
-    float top = 0.f, sum = 0.f;
     for (int k = threadIdx.y; k < 32; k += blockDim.y) {
         int x = x0 + threadIdx.x, y = y0 + k;
-        if (x < nx && y < ny) {
-            const T v = src[(size_t)y * nx + x];
-            tile[k][threadIdx.x] = v;
-            const float m = fabsf((float)v);
-            top = fmaxf(top, m <= FLT_MAX ? m : INFINITY);
-            sum += m;
-        }
-    }
-    if (stats) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-            sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        }
-        if (threadIdx.x == 0) s_red[threadIdx.y] = make_float2(top, sum);
+        if (x < nx && y < ny) tile[k][threadIdx.x] = src[(size_t)y * nx + x];
     }
     __syncthreads();
-    if (stats && threadIdx.x == 0 && threadIdx.y == 0) {
-        for (int k = 1; k < (int)blockDim.y; ++k) {
-            top = fmaxf(top, s_red[k].x);
-            sum += s_red[k].y;
-        }
-        stats[(slice * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = make_float2(top, sum);
-    }
     for (int k = threadIdx.y; k < 32; k += blockDim.y) {
         int y = y0 + threadIdx.x, x = x0 + k;
         if (x < nx && y < ny) dst[(size_t)x * ny + y] = tile[threadIdx.x][k];
@@ -890,85 +862,6 @@ __device__ __forceinline__ void fp_line(LineBase L, float t, float W, float Cm, 
     }
 }
 
-// Fixed-point tables, parallel beams.  F only enters through the differences of
-// neighbouring edges' sums over lines, so a common step q for a slice serves as
-// well as a floating exponent: entry i holds rint(M_i / q) modulo 2^32 and the
-// cell value r_i, 8 bytes read at once instead of 8 and 4, and the sums over
-// kFoldLines lines are integers whose differences are exact as long as a cell's
-// sum over those lines is below 2^31 q.  The differences are then added at 2^shift
-// q (fp_fold_fixed).  With q = room max 2^-31 (room: a cell's footprint times
-// kFoldLines) an entry is rounded to 2e-8 of the largest pixel for cells of one
-// pixel, 10 times finer than the FP32 fraction of the lookup position rounds
-// the interpolation, and the differences of 512 lines to 6e-7.  Slices whose
-// values are not finite or whose largest pixel is more than kFixedRange times
-// the mean, where a step in proportion to the largest would cost the small ones
-// bits, keep the FP64 tables (slice_step).
-//
-// The sweep is bound by shared-memory wavefronts: one 8-byte read per lookup
-// instead of an 8- and a 4-byte one, and no FP64 add.  16 slices of 512 x 512, 720
-// views of 768 cells: 2.82 -> 2.25 ms, the error against 64 bits unchanged
-// (1.2e-7).  Without the folds (a step 32 times coarser) 2.12 ms, but 1.3e-7.
-// Fan beams gain 3% (their line weights take a 64-bit multiply-add either way)
-// and stay with FP64 tables.
-constexpr float kFixedRange = 16.f;
-constexpr int kFoldLines = 16;
-__host__ __device__ __forceinline__ size_t line_bytes_fixed(int n) { return (size_t)8 * line_nf(n); }
-
-// The step q of a slice from the statistics of its tiles (0: FP64 tables).
-// room: largest multiple of a pixel that a sum must hold.
-__device__ __forceinline__ float slice_step(const float2* __restrict__ stats, int ntiles, float npx, float room,
-                                            int lane) {
-    float top = 0.f, sum = 0.f;
-    for (int i = lane; i < ntiles; i += 32) {
-        const float2 v = stats[i];
-        top = fmaxf(top, v.x);
-        sum += v.y;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-        sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    }
-    if (top == 0.f) return 1.f;
-    if (!(top >= 1e-25f && top <= 1e30f) || !(top * npx <= kFixedRange * sum)) return 0.f;
-    return room * top * 4.656612873e-10f;  // 2^-31
-}
-
-__device__ __forceinline__ void lds_entry(unsigned addr, int& m, float& r) {
-    asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(m), "=f"(r) : "r"(addr));
-}
-
-// fp_line of a parallel beam on a fixed-point table at base (line_base's f).
-template <int NI>
-__device__ __forceinline__ void fp_line_fixed(unsigned base, float tau, float W, float Cm, const float (&A)[NI],
-                                              const float (&B)[NI], unsigned (&acc)[NI], float (&alo)[NI]) {
-#pragma unroll
-    for (int q = 0; q < NI; ++q) {
-        const float xn = fma_sat(B[q], tau, A[q]);
-        const float tt = fmaf(xn, W, Cm);
-        int m;
-        float r;
-        lds_entry(base + 8u * __float_as_uint(tt), m, r);
-        acc[q] += (unsigned)m;
-        alo[q] = fmaf(r, fmaf(xn, W, Cm - tt), alo[q]);
-    }
-}
-
-// At most kFoldLines lines' sums and FP32 parts (scale: steps per FP32 unit):
-// the difference to the next edge's, exact modulo 2^32, joins the cell's sum.
-template <int NI>
-__device__ __forceinline__ void fp_fold_fixed(unsigned (&acc)[NI], float (&alo)[NI], int (&sum)[NI], float scale,
-                                              int shift) {
-    const int half = (1 << shift) >> 1;
-#pragma unroll
-    for (int q = 0; q < NI; ++q) {
-        const unsigned a = acc[q] + (unsigned)__float2int_rn(alo[q] * scale);
-        sum[q] += ((int)(__shfl_down_sync(0xffffffffu, a, 1) - a) + half) >> shift;
-        acc[q] = 0;
-        alo[q] = 0.f;
-    }
-}
-
 // Fold the FP32 parts (at most 16 lines of r * frac) into the FP64 sums.
 template <int NI>
 __device__ __forceinline__ void fp_renorm(double (&accd)[NI], float (&alo)[NI]) {
@@ -1063,74 +956,26 @@ __host__ __device__ __forceinline__ size_t line_tables_warp_bytes(int n) {
     return line_bytes(n) + (((size_t)n * 4 + 15) & ~(size_t)15);
 }
 
-// Fixed-point midpoint table of one line (build_line_fp64's entries, M / q
-// rounded to an integer modulo 2^32), sums in FP64.
-template <typename Cell>
-__device__ __forceinline__ void build_line_fixed(unsigned char* __restrict__ line, int n, int lane, float q, Cell cell) {
-    int2* E2 = reinterpret_cast<int2*>(line);
-    const double inv = 1.0 / (double)q;
-    const int ne = n + 2;
-    const int E = (ne + 31) / 32;
-    const int k0 = lane * E;
-    double tot = 0.0;
-    for (int p = 0; p < E; ++p) {
-        const int i = k0 + p - 1;
-        if (i >= 0 && i < n) tot += (double)cell(i);
-    }
-    double inc = tot;  // inclusive scan of the lane totals
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const double t = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += t;
-    }
-    double c = inc - tot;
-    for (int p = 0; p < E; ++p) {
-        const int k = k0 + p, i = k - 1;
-        if (k < ne) {
-            const float r = (i >= 0 && i < n) ? cell(i) : 0.f;
-            E2[k] = make_int2((int)__double2ll_rn((c + 0.5 * (double)r) * inv), __float_as_int(r));
-            c += (double)r;
-        }
-    }
-    if (ne + lane < line_nf(n)) E2[ne + lane] = make_int2(0, 0);
-}
-
-// The tables of every line of a stack of slices (one warp per line, blockIdx.y
-// the slice), for the forward projector that streams them into shared memory.
-// The warp reads the line's cells into shared memory with coalesced loads,
-// builds the table there (each lane scans a run of consecutive entries) and
-// writes it out with coalesced 16-byte stores.  A slice's tables start at
-// slice * nl * line_bytes(n) in either form.  step[slice] (null: FP64 tables)
-// is the fixed-point step, 0 for FP64; with stats the launch finds it from the
-// tiles' statistics, without it reads what an earlier launch found.
+// The tables of every line of a stack of slices (one warp per line), for the
+// forward projector that streams them into shared memory.  The warp reads the
+// line's cells into shared memory with coalesced loads, builds the table
+// there (each lane scans a run of consecutive entries) and writes it out with
+// coalesced 16-byte stores.
 template <typename Tin>
 __global__ void __launch_bounds__(256) line_tables_kernel(unsigned char* __restrict__ out,
-                                                          const Tin* __restrict__ src, int nl, int n,
-                                                          float* __restrict__ step, const float2* __restrict__ stats,
-                                                          int ntiles, float room) {
+                                                          const Tin* __restrict__ src, long long nlines, int n) {
     extern __shared__ float4 s_lt4[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const size_t slice = blockIdx.y;
-    float q = 0.f;
-    if (step) {
-        if (stats) {
-            q = slice_step(stats + slice * ntiles, ntiles, (float)nl * (float)n, room, lane);
-            if (blockIdx.x == 0 && threadIdx.x == 0) step[slice] = q;
-        } else {
-            q = step[slice];
-        }
-    }
-    const size_t lb = q > 0.f ? line_bytes_fixed(n) : line_bytes(n);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const size_t lb = line_bytes(n);
     unsigned char* tab = reinterpret_cast<unsigned char*>(s_lt4) + warp * line_tables_warp_bytes(n);
-    float* cells = reinterpret_cast<float*>(tab + line_bytes(n));
-    out += slice * nl * line_bytes(n);
-    src += slice * nl * n;
-    for (int l = blockIdx.x * nwarps + warp; l < nl; l += gridDim.x * nwarps) {
-        const Tin* row = src + (size_t)l * n;
+    float* cells = reinterpret_cast<float*>(tab + lb);
+    const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+    for (long long l = w0; l < nlines; l += nw) {
+        const Tin* row = src + l * n;
         for (int i = lane; i < n; i += 32) cells[i] = ldf(row + i);
         __syncwarp();
-        if (q > 0.f) build_line_fixed(tab, n, lane, q, [&](int i) { return cells[i]; });
-        else build_line_fp64(tab, n, lane, [&](int i) { return cells[i]; });
+        build_line_fp64(tab, n, lane, [&](int i) { return cells[i]; });
         __syncwarp();
         const uint4* from = reinterpret_cast<const uint4*>(tab);
         uint4* to = reinterpret_cast<uint4*>(out + l * lb);
@@ -1303,19 +1148,15 @@ __device__ unsigned int g_first_wait_polls = kWaitPolls;
 
 // Above 8 edge groups per warp (five or six registers per group) two CTAs
 // per SM.
-template <bool FAN, int NI, bool FIXED>
-constexpr int fp_stream_min_blocks() { return NI <= (FIXED ? 12 : 8) ? 3 : 2; }
+template <bool FAN, int NI>
+constexpr int fp_stream_min_blocks() { return NI <= 8 ? 3 : 2; }
 
-template <bool FAN, int NI, bool FIXED, typename Tout>
-__global__ void __launch_bounds__(256, (fp_stream_min_blocks<FAN, NI, FIXED>())) dd2d_fp_stream_kernel(Tout* __restrict__ prj, const unsigned char* __restrict__ ltab0,
+template <bool FAN, int NI, typename Tout>
+__global__ void __launch_bounds__(256, (fp_stream_min_blocks<FAN, NI>())) dd2d_fp_stream_kernel(Tout* __restrict__ prj, const unsigned char* __restrict__ ltab0,
                                                              const unsigned char* __restrict__ ltab1, DDTab tab, Grid g,
-                                                             Det d, int nview, int vgroup, int wpv, int ring_lines, int slice0,
+                                                             Det d, int nview, int vgroup, int wpv, int rchunk, int slice0,
                                                              const int* __restrict__ order, const float* __restrict__ deg,
-                                                             int unweight_par, const float* __restrict__ step, int shift) {
-    // a slice's tables are fixed-point or FP64 (line_tables_kernel); this launch
-    // takes the slices of its own kind
-    const float unit = step ? step[blockIdx.x] : 0.f;
-    if ((unit > 0.f) != FIXED) return;
+                                                             int unweight_par) {
     extern __shared__ float4 s_ring4[];  // [2][rchunk line tables of max(nx, ny) cells]
     unsigned char* s_ring = reinterpret_cast<unsigned char*>(s_ring4);
     __shared__ __align__(8) unsigned long long s_bar[2];
@@ -1328,10 +1169,7 @@ __global__ void __launch_bounds__(256, (fp_stream_min_blocks<FAN, NI, FIXED>()))
     const int slice = slice0 + (int)blockIdx.x;
     const int iz = slice % g.nz, b = slice / g.nz;
     const int ipv = (d.nu + 30) / 31;  // edge groups per view
-    const size_t ring = (size_t)ring_lines * line_bytes(max(g.nx, g.ny));  // bytes per buffer
-    auto table_bytes = [](int n) { return FIXED ? line_bytes_fixed(n) : line_bytes(n); };
-    // lines per buffer (fixed-point tables are smaller)
-    const int rchunk = FIXED ? min(8, (int)(ring / line_bytes_fixed(max(g.nx, g.ny)))) : ring_lines;
+    const size_t ring = (size_t)rchunk * line_bytes(max(g.nx, g.ny));  // bytes per buffer
 
     // orientations with work in this CTA: rows (o = 0) for views traced along
     // y, columns (o = 1) for views traced along x, both in the blend band
@@ -1354,10 +1192,10 @@ __global__ void __launch_bounds__(256, (fp_stream_min_blocks<FAN, NI, FIXED>()))
         const int c = o == 0 ? k : k - nc0;
         const int n = o == 0 ? g.nx : g.ny, nl = o == 0 ? g.ny : g.nx;
         const int l0 = c * rchunk, nlc = min(rchunk, nl - l0);
-        const unsigned bytes = (unsigned)((size_t)nlc * table_bytes(n));
+        const unsigned bytes = (unsigned)((size_t)nlc * line_bytes(n));
         unsigned long long* bar = &s_bar[k & 1];
         mbar_expect_tx(bar, bytes);
-        bulk_copy_g2s(s_ring + (k & 1) * ring, (o == 0 ? src0 : src1) + (size_t)l0 * table_bytes(n), bytes, bar);
+        bulk_copy_g2s(s_ring + (k & 1) * ring, (o == 0 ? src0 : src1) + (size_t)l0 * line_bytes(n), bytes, bar);
     };
     if (threadIdx.x == 0) {
         mbar_init(&s_bar[0], 1);
@@ -1372,9 +1210,7 @@ __global__ void __launch_bounds__(256, (fp_stream_min_blocks<FAN, NI, FIXED>()))
 
     // per edge group: edge position and slope, and the sums of fp_line
     float A[NI], B[NI], S[NI], alo[NI];
-    std::conditional_t<FIXED, unsigned, double> accd[NI];
-    int cell[NI];  // fixed-point: the cells' sums (fp_fold_fixed)
-    const float fold = FIXED ? 1.f / unit : 0.f;
+    double accd[NI];
     const int renorm = max(1, 16 / rchunk);  // chunks between renormalisations of (acc, alo)
     const unsigned first_polls = g_first_wait_polls;
     bool failed = false;
@@ -1394,8 +1230,7 @@ __global__ void __launch_bounds__(256, (fp_stream_min_blocks<FAN, NI, FIXED>()))
                 A[q] = 0.5f;
                 B[q] = 0.f;
                 S[q] = 0.5f;
-                accd[q] = 0;
-                if (FIXED) cell[q] = 0;
+                accd[q] = 0.0;
                 alo[q] = 0.f;
                 if (vi < nvg && m < ipv) {
                     const int view = order[v0 + vi];
@@ -1419,29 +1254,17 @@ __global__ void __launch_bounds__(256, (fp_stream_min_blocks<FAN, NI, FIXED>()))
         const float W = (float)(n + 1), Cm = kRoundMagic - 1.f;
         float tl = (float)(l0 - anchor);  // line coordinate, stepped exactly
         LineBase L = line_base(buf, n);
-        const unsigned lb = (unsigned)table_bytes(n);
-        for (int r = 0; r < nlc && !failed; ++r, tl += 1.f, L.f += lb, L.r += lb) {
-            if constexpr (FIXED) fp_line_fixed<NI>(L.f, tl, W, Cm, A, B, accd, alo);
-            else fp_line<FAN, NI>(L, tl, W, Cm, A, B, S, accd, alo);
-        }
-        if ((c + 1) % renorm == 0 || c == last) {
-            if constexpr (FIXED) fp_fold_fixed<NI>(accd, alo, cell, fold, shift);
-            else fp_renorm<NI>(accd, alo);
-        }
+        const unsigned lb = (unsigned)line_bytes(n);
+        for (int r = 0; r < nlc && !failed; ++r, tl += 1.f, L.f += lb, L.r += lb)
+            fp_line<FAN, NI>(L, tl, W, Cm, A, B, S, accd, alo);
+        if ((c + 1) % renorm == 0 || c == last) fp_renorm<NI>(accd, alo);
         if (c == last && !failed) {
 #pragma unroll
             for (int q = 0; q < NI; ++q) {
                 int vi, m;
                 fp_item(warp, q, ipv, wpv, vi, m);
                 if (vi >= nvg || m >= ipv) continue;
-                float sum;
-                if constexpr (FIXED) {
-                    const float An = __shfl_down_sync(0xffffffffu, A[q], 1);
-                    sum = __fdividef((float)((double)cell[q] * (double)unit * (double)(1 << shift)), An - A[q]);
-                } else {
-                    sum = fp_cell_sum(accd[q], FAN ? B[q] : A[q]);
-                }
-                sum /= (float)(n + 1);
+                const float sum = fp_cell_sum(accd[q], FAN ? B[q] : A[q]) / (float)(n + 1);
                 const int view = order[v0 + vi];
                 const int kk = 31 * m + lane;
                 const float wx = tab.wx[view];
@@ -1694,9 +1517,9 @@ int launch_fp(void* prj, const void* img, const float* deg, const ctp_geometry& 
     if (rc) return rc;
     Tin* imgT = reinterpret_cast<Tin*>(ws + fp_edge_table_bytes(g));
     const size_t slice_px = g.ny * g.nx;
-    auto transpose = [&](const Tin* from, int nsl, float2* stats) {
+    auto transpose = [&](const Tin* from, int nsl) {
         dim3 tg((unsigned)((g.nx + 31) / 32), (unsigned)((g.ny + 31) / 32), (unsigned)nsl);
-        transpose_kernel<Tin><<<tg, dim3(32, 8), 0, s>>>(imgT, from, (int)g.nx, (int)g.ny, stats);
+        transpose_kernel<Tin><<<tg, dim3(32, 8), 0, s>>>(imgT, from, (int)g.nx, (int)g.ny);
         return check_launch("transpose_kernel");
     };
     int unweight = (geom == 1) && (type & CTP_TYPE_FORCE_FBP);
@@ -1743,33 +1566,15 @@ int launch_fp(void* prj, const void* img, const float* deg, const ctp_geometry& 
         size_t shm = 2 * (size_t)rc_s * line_bytes((int)std::max(g.nx, g.ny));
         const bool fan = geom == 0;
         const int wpv = fan ? 8 / sv : 0;  // fan beams: warps per view (fp_item)
-        // parallel beams, fixed-point tables: the slices' steps go where the edge
-        // table holds the fan source's positions, the tiles' statistics where the
-        // column tables come afterwards
-        DDTabW tw;
-        carve_table(reinterpret_cast<float*>(ws), g.nview, g.nu, tw);
-        const int ntiles = (int)(((g.nx + 31) / 32) * ((g.ny + 31) / 32));
-        // a cell's footprint along a line, at most (views are swept along the axis
-        // within 50 degrees of the rays), over the lines of one fold
-        const double foot = 1.6 * fabs((double)g.du) / std::min((double)g.dx, (double)g.dy) + 1.0;
-        const double room = 1.05 * kFoldLines * foot;
-        int shift = 0;
-        while (((size_t)kFoldLines << shift) < std::max(g.nx, g.ny)) ++shift;
-        const bool fixed = !fan && (size_t)chunk <= 4 * g.nview && foot < 1e4 &&
-                           (size_t)ntiles * sizeof(float2) <= g.nx * line_bytes((int)g.ny);
-        float* step = fixed ? tw.sP[0] : nullptr;
         for (int s0 = 0; s0 < nslices; s0 += chunk) {
             const int cs = std::min(chunk, nslices - s0);
             const Tin* from = cptr<Tin>(img) + (size_t)s0 * slice_px;
-            float2* stats = fixed ? reinterpret_cast<float2*>(lt1) : nullptr;
-            if ((rc = transpose(from, cs, stats))) return rc;
-            auto blocks = [&](size_t lines) {
-                return (unsigned)std::min<size_t>((lines + lt_warps - 1) / lt_warps, std::max(1, 148 * 8 / cs));
-            };
-            line_tables_kernel<Tin><<<dim3(blocks(g.ny), (unsigned)cs), 32 * lt_warps, lt_shm, s>>>(
-                lt0, from, (int)g.ny, (int)g.nx, step, stats, ntiles, (float)room);
-            line_tables_kernel<Tin><<<dim3(blocks(g.nx), (unsigned)cs), 32 * lt_warps, lt_shm, s>>>(
-                lt1, imgT, (int)g.nx, (int)g.ny, step, nullptr, 0, 0.f);
+            if ((rc = transpose(from, cs))) return rc;
+            const long long rows = (long long)cs * g.ny, cols = (long long)cs * g.nx;
+            const unsigned rgrid = (unsigned)std::min<long long>((rows + lt_warps - 1) / lt_warps, 148 * 8);
+            const unsigned cgrid = (unsigned)std::min<long long>((cols + lt_warps - 1) / lt_warps, 148 * 8);
+            line_tables_kernel<Tin><<<rgrid, 32 * lt_warps, lt_shm, s>>>(lt0, from, rows, (int)g.nx);
+            line_tables_kernel<Tin><<<cgrid, 32 * lt_warps, lt_shm, s>>>(lt1, imgT, cols, (int)g.ny);
             if ((rc = check_launch("line_tables_kernel"))) return rc;
             // slices along x, view groups along y: CTAs are dispatched view
             // group by view group, the blend band's first
@@ -1778,21 +1583,15 @@ int launch_fp(void* prj, const void* img, const float* deg, const ctp_geometry& 
                 cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
                 cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
                 kern<<<fg, 256, shm, s>>>(mptr<Tout>(prj), lt0, lt1, tab, make_grid(g), make_det(g), (int)g.nview,
-                                          sv, wpv, rc_s, s0, order, deg, unweight, step, shift);
+                                          sv, wpv, rc_s, s0, order, deg, unweight);
             };
-#define CTP_FP_STREAM(FAN_, FIXED_)                                           \
-    if (ni == 4) launch(dd2d_fp_stream_kernel<FAN_, 4, FIXED_, Tout>);        \
-    else if (ni == 8) launch(dd2d_fp_stream_kernel<FAN_, 8, FIXED_, Tout>);   \
-    else if (ni == 12) launch(dd2d_fp_stream_kernel<FAN_, 12, FIXED_, Tout>); \
-    else launch(dd2d_fp_stream_kernel<FAN_, 16, FIXED_, Tout>)
-            if (fixed) {
-                CTP_FP_STREAM(false, true);
-            }
-            if (fan) {
-                CTP_FP_STREAM(true, false);
-            } else {
-                CTP_FP_STREAM(false, false);
-            }
+#define CTP_FP_STREAM(NI_)                                                       \
+    if (fan) launch(dd2d_fp_stream_kernel<true, NI_, Tout>);                     \
+    else launch(dd2d_fp_stream_kernel<false, NI_, Tout>)
+            if (ni == 4) { CTP_FP_STREAM(4); }
+            else if (ni == 8) { CTP_FP_STREAM(8); }
+            else if (ni == 12) { CTP_FP_STREAM(12); }
+            else { CTP_FP_STREAM(16); }
 #undef CTP_FP_STREAM
             if ((rc = check_launch("dd2d_fp_stream_kernel"))) return rc;
         }
@@ -1802,7 +1601,7 @@ int launch_fp(void* prj, const void* img, const float* deg, const ctp_geometry& 
     if (ws_bytes < fp_workspace_min(g))
         return set_error(CTP_ERR_INVALID_ARGUMENT, "dd2d_fp: workspace of %zu bytes, the kernel needs %zu", ws_bytes,
                          fp_workspace_min(g));
-    if ((rc = transpose(cptr<Tin>(img), nslices, nullptr))) return rc;
+    if ((rc = transpose(cptr<Tin>(img), nslices))) return rc;
     if (shaped) {
         size_t shm = (size_t)nrows * line_bytes((int)std::max(g.nx, g.ny));
         dim3 fg((unsigned)((g.nview + sv - 1) / sv), (unsigned)(g.nbatch * g.nz));

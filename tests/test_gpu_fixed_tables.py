@@ -1,6 +1,7 @@
-"""Parallel forward projection from fixed-point line tables at the sizes where
-they can go wrong: lines around one fold, cells much finer and coarser than the
-pixels, and slices of every kind of value in one call."""
+"""Parallel forward projection at the sizes where its line tables can go wrong:
+lines around sixteen (the FP32 parts' renormalisation), cells much finer and
+coarser than the pixels, slices of every kind of value in one call, and faint
+regions beside bright ones."""
 import numpy as np
 import pytest
 
@@ -12,8 +13,7 @@ torch = pytest.importorskip("torch")
 # Per line the lookup position is rounded to 2^-25 of the line, n 2^-25 pixels:
 # over n lines of values of the image's size, relative to a ray sum of n times
 # the cell's width w in pixels, n 2^-25 sqrt(2 n) / (n w) = 2^-25 sqrt(2 n) / w:
-# 9e-7 at n = 300 and w = 1; the entries' rounding (2e-8 of the largest pixel)
-# is below that.  Narrow cells (w = 0.2) lose the same five times.
+# 9e-7 at n = 300 and w = 1.  Narrow cells (w = 0.2) lose the same five times.
 TOL = 1.5e-6
 
 
@@ -49,7 +49,7 @@ def test_lines_and_cells(nx, ny, nu, width, nbatch, oracle):
 
 
 def test_slices_of_every_kind(oracle):
-    """Each slice takes the tables that its own values allow."""
+    """Scales, signs, a dominant pixel and zeros, each slice by itself."""
     p, ang = scan(97, 83, 140, 1.0)
     rng = np.random.default_rng(7)
     x = rng.uniform(0, 1, (9, 1, 83, 97)).astype(np.float32)
@@ -57,8 +57,8 @@ def test_slices_of_every_kind(oracle):
     x[2] *= 1e-18
     x[3] *= 1e18
     x[4] *= -1
-    x[5, 0, 40, 40] = 3e4       # largest over mean beyond the fixed-point range
-    x[6, 0, :40] = 0            # and within it
+    x[5, 0, 40, 40] = 3e4       # one pixel far above the mean
+    x[6, 0, :40] = 0
     out = fp(p, x, ang)
     ref = oracle.dd_fp(p, x, ang, "parallel")
     assert not out[1].any()
@@ -83,3 +83,23 @@ def test_storage(dtype, oracle):
     ref = oracle.dd_fp(p, x, ang, "parallel")
     # the stored result rounds to 2^-9 (bfloat16) or 2^-12 (float16) at most
     assert rel_l2(fp(p, x, ang, dt), ref) <= (2.0**-9 if dtype == "bfloat16" else 2.0**-12) + TOL
+
+
+def test_faint_half_keeps_its_own_precision(oracle):
+    """Rays that meet only the faint half of a slice (1e-4 of the bright one)
+    are as exact, ray by ray, as those of a slice without a bright half."""
+    n = 300
+    p, ang = scan(n, n, 300, 1.0, nview=3)
+    ang = np.array([0.011, 0.02, 3.13], np.float32)
+    rng = np.random.default_rng(11)
+    x = (1e-4 * rng.uniform(0, 1, (1, 1, n, n))).astype(np.float32)
+    bright = np.zeros_like(x)
+    bright[..., : n // 2] = rng.uniform(0.5, 1, (1, 1, n, n // 2))
+    x += bright
+    faint = oracle.dd_fp(p, bright, ang, "parallel") == 0
+    ref = oracle.dd_fp(p, x, ang, "parallel")
+    faint &= ref > 0.1 * n * 0.5e-4
+    assert faint.sum() > 200
+    out = fp(p, x, ang)
+    # TOL is the root mean square over rays: four times that for the worst of some hundred
+    assert (np.abs(out - ref)[faint] / ref[faint]).max() <= 4 * TOL
