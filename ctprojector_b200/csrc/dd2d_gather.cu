@@ -11,16 +11,18 @@
 //   pixel   the pixel-driven back projection (bpFanKernel3D fbp.cu:265-337 with
 //           the FBP distance weight, bpParallelKernel3D fbpParallel.cu:200-250):
 //           the detector row interpolated linearly at the pixel's centre
-// The first three are differences of F, the running integral of a detector row, at
+// The mean is a difference of F, the running integral of a detector row, at
 // the detector coordinates j of the pixel's two edges: (F(j1) - F(j0)) /
-// (j1 - j0) for the mean, and F(j1) - F(j0) for the transpose: the forward
+// (j1 - j0).  The transpose is the integral from j0 to j1 too: the forward
 // projector spreads cell k over the interval between its edge rays on the
 // pixel's line, so the pixel's share of the cell is the overlap of [j0, j1]
-// with [k, k + 1].  For parallel beams j is linear along the line.  For fan
-// beams the edge rays sit at angles k du while the forward projector's cells
-// are linear in position; with f the fraction of the cell in angle and T the
-// tangent of the ray's angle to the line's normal, sin and cos addition
-// theorems give the fraction in position
+// with [k, k + 1].  It is added up cell by cell, not as a difference of F: a
+// gradient may hold cells of any size, or that are not finite, and they count
+// for the pixels that they meet alone.  For parallel beams j is linear along
+// the line.  For fan beams the edge rays sit at angles k du while the forward
+// projector's cells are linear in position; with f the fraction of the cell in
+// angle and T the tangent of the ray's angle to the line's normal, sin and cos
+// addition theorems give the fraction in position
 //   f + f (1 - f) (du T + du^2 (2 f - 1) / 3) + O(du^3).
 //
 // A sweep is one view with one kind of edge: the pixels' x-edges (views traced
@@ -142,6 +144,12 @@ __device__ __forceinline__ void lds_entry(unsigned addr, f32x2& m, f32x2& v) {
 __device__ __forceinline__ void lds_entry(unsigned addr, float& m, float& v) {
     asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(m), "=f"(v) : "r"(addr));
 }
+__device__ __forceinline__ void lds_value(unsigned addr, f32x2& v) {
+    asm volatile("ld.shared.u64 %0, [%1];" : "=l"(v) : "r"(addr));
+}
+__device__ __forceinline__ void lds_value(unsigned addr, float& v) {
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+}
 
 // Midpoint tables of two detector rows, staged by one warp: entries k = 0 ..
 // win of (running sum of the window cells before k + value / 2, value) for the
@@ -151,28 +159,45 @@ __device__ __forceinline__ void lds_entry(unsigned addr, float& m, float& v) {
 // weights of the cells.
 template <typename Tp>
 struct RowItem {
-    const Tp* row;    // null: zeros
+    const Tp* row;    // null: `off` for every cell
     const float* lw;  // weights of the row's cells, or null
     int w0;
+    float off;        // value of cells off the detector
+    float scale;      // of the values (adjoint)
 };
 
-// LINEAR: entries (value of cell k, step to cell k + 1; the last cell steps by
-// zero) for linear interpolation instead.
-template <int PER, bool PAIR, bool LINEAR, typename Tp>
+// kGatherPixel: entries (value of cell k, step to cell k + 1; the last cell steps
+// by zero) for linear interpolation instead.  kGatherAdjoint: the values alone,
+// lane l those of k = l, l + 32, ...
+template <int PER, bool PAIR, int MODE, typename Tp>
 __device__ __forceinline__ void stage_rows_per(const RowItem<Tp> (&it)[2], float* t0, float* t1, int win, int nu,
                                                int lane) {
-    const int k0 = lane * PER;
+    constexpr int kNext = MODE == kGatherAdjoint ? 32 : 1;
+    const int k0 = MODE == kGatherAdjoint ? lane : lane * PER;
     float v[2][PER], run[2], incl[2];
 #pragma unroll
     for (int m = 0; m < 2; ++m)
 #pragma unroll
         for (int q = 0; q < PER; ++q) {
-            const int k = k0 + q, cell = it[m].w0 + k;
+            const int k = k0 + q * kNext, cell = it[m].w0 + k;
             const bool in = it[m].row && k < win && cell >= 0 && cell < nu;
-            v[m][q] = in ? ldf(it[m].row + cell) : 0.f;
-            if (it[m].lw) v[m][q] *= in ? __ldg(it[m].lw + cell) : 0.f;
+            v[m][q] = in ? ldf(it[m].row + cell) : it[m].off;
+            if (it[m].lw && in) v[m][q] *= __ldg(it[m].lw + cell);
+            if (MODE == kGatherAdjoint) v[m][q] *= it[m].scale;
         }
-    if constexpr (LINEAR) {
+    if constexpr (MODE == kGatherAdjoint) {
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            const int k = k0 + q * kNext;
+            if (k > win) continue;
+            if constexpr (PAIR) {
+                reinterpret_cast<float2*>(t0)[k] = make_float2(v[0][q], v[1][q]);
+            } else {
+                t0[k] = v[0][q];
+                if (t1) t1[k] = v[1][q];
+            }
+        }
+    } else if constexpr (MODE == kGatherPixel) {
 #pragma unroll
         for (int q = 0; q < PER; ++q) {
             const int k = k0 + q;
@@ -225,17 +250,17 @@ __device__ __forceinline__ void stage_rows_per(const RowItem<Tp> (&it)[2], float
     }
 }
 
-template <bool PAIR, bool LINEAR, typename Tp>
+template <bool PAIR, int MODE, typename Tp>
 __device__ __forceinline__ void stage_rows(const RowItem<Tp> (&it)[2], float* t0, float* t1, int win, int nu, int lane) {
     switch ((win + 1 + 31) / 32) {
-        case 1: stage_rows_per<1, PAIR, LINEAR>(it, t0, t1, win, nu, lane); break;
-        case 2: stage_rows_per<2, PAIR, LINEAR>(it, t0, t1, win, nu, lane); break;
-        case 3: stage_rows_per<3, PAIR, LINEAR>(it, t0, t1, win, nu, lane); break;
-        case 4: stage_rows_per<4, PAIR, LINEAR>(it, t0, t1, win, nu, lane); break;
-        case 5: stage_rows_per<5, PAIR, LINEAR>(it, t0, t1, win, nu, lane); break;
-        case 6: stage_rows_per<6, PAIR, LINEAR>(it, t0, t1, win, nu, lane); break;
-        case 7: stage_rows_per<7, PAIR, LINEAR>(it, t0, t1, win, nu, lane); break;
-        default: stage_rows_per<8, PAIR, LINEAR>(it, t0, t1, win, nu, lane); break;
+        case 1: stage_rows_per<1, PAIR, MODE>(it, t0, t1, win, nu, lane); break;
+        case 2: stage_rows_per<2, PAIR, MODE>(it, t0, t1, win, nu, lane); break;
+        case 3: stage_rows_per<3, PAIR, MODE>(it, t0, t1, win, nu, lane); break;
+        case 4: stage_rows_per<4, PAIR, MODE>(it, t0, t1, win, nu, lane); break;
+        case 5: stage_rows_per<5, PAIR, MODE>(it, t0, t1, win, nu, lane); break;
+        case 6: stage_rows_per<6, PAIR, MODE>(it, t0, t1, win, nu, lane); break;
+        case 7: stage_rows_per<7, PAIR, MODE>(it, t0, t1, win, nu, lane); break;
+        default: stage_rows_per<8, PAIR, MODE>(it, t0, t1, win, nu, lane); break;
     }
 }
 
@@ -244,7 +269,7 @@ __device__ __forceinline__ void stage_rows(const RowItem<Tp> (&it)[2], float* t0
 template <int S>
 struct Lanes {
     static constexpr int NP = S / 2;       // pairs
-    static constexpr int kEntry = 16;      // bytes of a table entry
+    static constexpr int kEntry = 16;      // bytes of a table entry (the adjoint's: half of it)
     f32x2 a[NP][4];
     __device__ __forceinline__ void zero() {
 #pragma unroll
@@ -277,6 +302,29 @@ struct Lanes {
 #pragma unroll
         for (int q = 0; q < NP; ++q) a[q][k] = fma2(p.f[q], w2, a[q][k]);
     }
+    // every slice's value of the cell at addr
+    __device__ __forceinline__ static Point value(unsigned addr, unsigned plane) {
+        Point p;
+#pragma unroll
+        for (int q = 0; q < NP; ++q) lds_value(addr + q * plane, p.f[q]);
+        return p;
+    }
+    __device__ __forceinline__ static Point zero_point() {
+        Point p;
+#pragma unroll
+        for (int q = 0; q < NP; ++q) p.f[q] = 0ull;
+        return p;
+    }
+    __device__ __forceinline__ static void scale_add(Point& t, const Point& v, float w) {
+        const f32x2 w2 = pack2(w, w);
+#pragma unroll
+        for (int q = 0; q < NP; ++q) t.f[q] = fma2(v.f[q], w2, t.f[q]);
+    }
+    __device__ __forceinline__ void add(int k, const Point& t) {
+        const f32x2 one = pack2(1.f, 1.f);
+#pragma unroll
+        for (int q = 0; q < NP; ++q) a[q][k] = fma2(t.f[q], one, a[q][k]);
+    }
     __device__ __forceinline__ float get(int s, int k) const {
         float x, y;
         unpack2(a[s / 2][k], x, y);
@@ -306,6 +354,14 @@ struct Lanes<1> {
         a[k] = fmaf(hi.f - lo.f, w, a[k]);
     }
     __device__ __forceinline__ void add(int k, const Point& p, float w) { a[k] = fmaf(p.f, w, a[k]); }
+    __device__ __forceinline__ static Point value(unsigned addr, unsigned) {
+        Point p;
+        lds_value(addr, p.f);
+        return p;
+    }
+    __device__ __forceinline__ static Point zero_point() { return Point{0.f}; }
+    __device__ __forceinline__ static void scale_add(Point& t, const Point& v, float w) { t.f = fmaf(v.f, w, t.f); }
+    __device__ __forceinline__ void add(int k, const Point& t) { a[k] += t.f; }
     __device__ __forceinline__ float get(int, int k) const { return a[k]; }
     __device__ __forceinline__ void set(int, int k, float x, float) { a[k] = x; }
 };
@@ -346,10 +402,14 @@ __device__ __forceinline__ void store_out(void* img, size_t i, float v, int lp, 
     }
 }
 
+// Bytes of a table entry: two numbers per slice, for the adjoint one.
+template <int MODE, int S>
+constexpr int entry_bytes() { return MODE == kGatherAdjoint ? Lanes<S>::kEntry / 2 : Lanes<S>::kEntry; }
+
 // Bytes of a CTA's dynamic shared memory: the tables of a chunk and the tile's sums.
-template <int S>
+template <int MODE, int S>
 size_t gather_smem(int win) {
-    const size_t tab = (size_t)Lanes<S>::NP * Lanes<S>::kEntry * kChunk * (win + 1);
+    const size_t tab = (size_t)Lanes<S>::NP * entry_bytes<MODE, S>() * kChunk * (win + 1);
     const size_t acc = (size_t)S * kT * (kT + 1) * sizeof(float);
     return tab + acc;
 }
@@ -365,7 +425,8 @@ __global__ void __launch_bounds__(256, (S == 4 ? 3 : 4)) gather_bp_kernel(const 
     const Grid& g = A.g;
     const Det& d = A.d;
     const int stride = A.win + 1;
-    const unsigned plane = kChunk * stride * L::kEntry;  // bytes of one pair's tables
+    constexpr int kEntry = entry_bytes<MODE, S>();
+    const unsigned plane = kChunk * stride * kEntry;  // bytes of one pair's tables
     float* tab = reinterpret_cast<float*>(s_raw);
     float* s_sum = tab + L::NP * plane / 4;  // [S][kT][kT + 1]
     const int tiles_x = (g.nx + kT - 1) / kT;
@@ -404,7 +465,7 @@ __global__ void __launch_bounds__(256, (S == 4 ? 3 : 4)) gather_bp_kernel(const 
     acc.zero();
     for (int i = threadIdx.x; i < S * kT * (kT + 1); i += 256) s_sum[i] = 0.f;  // (barriers below)
     const int vb = blockIdx.z * A.vper, ve = min(A.nview, vb + A.vper);
-    const unsigned tab_addr = (unsigned)__cvta_generic_to_shared(tab) - L::kEntry * kMagicBits;
+    const unsigned tab_addr = (unsigned)__cvta_generic_to_shared(tab) - kEntry * kMagicBits;  // (wraps)
     const float idu = 1.f / d.du;
 
     for (int vs = vb; vs < ve; vs += kList) {
@@ -489,9 +550,12 @@ __global__ void __launch_bounds__(256, (S == 4 ? 3 : 4)) gather_bp_kernel(const 
                     if (ok) w0 = (int)floor(jmin) - 2;
                     T.jb = (float)(jref - w0 - 0.5);
                     if (!ok) {  // an angle that is not a number: so is the result (the lookups stay inside)
+                        const float step = 1.f / 4096;
                         T.jb = 1.f;
-                        T.jx = T.jy = T.bx = T.by = 0.f;
-                        T.gx = T.gy = 1.f;
+                        T.jx = T.jy = FAN ? step * d.du : step;
+                        T.bx = T.by = 0.f;
+                        T.gx = copysignf(1e6f, d.du);
+                        T.gy = -T.gx;
                         T.w = NAN;
                     }
                     s_tile[threadIdx.x] = T;
@@ -499,11 +563,18 @@ __global__ void __launch_bounds__(256, (S == 4 ? 3 : 4)) gather_bp_kernel(const 
                 }
                 __syncthreads();
                 // stage the tables: pairs of slices of a sweep, or (S = 1) pairs of sweeps
+                auto item = [&](RowItem<Tp>& it, const Tp* row, int vi) {
+                    const int w0 = s_w0[qt + vi], view = vs + list[q0 + vi];
+                    const bool ok = w0 != INT_MIN;
+                    it.row = row && ok ? row + (size_t)view * vstride : nullptr;
+                    it.lw = lw ? lw + (size_t)view * d.nu : nullptr;
+                    it.w0 = ok ? w0 : 0;
+                    it.off = ok ? 0.f : NAN;
+                    it.scale = MODE == kGatherAdjoint && !FAN ? fabsf(s_tile[qt + vi].w) : 1.f;
+                };
                 if constexpr (S >= 2) {
                     for (int i = warp; i < n * L::NP; i += 8) {
                         const int vi = i / L::NP, p = i - vi * L::NP;
-                        const int w0 = s_w0[qt + vi];
-                        const int view = vs + list[q0 + vi];
                         RowItem<Tp> it[2];
 #pragma unroll
                         for (int m = 0; m < 2; ++m) {
@@ -511,27 +582,20 @@ __global__ void __launch_bounds__(256, (S == 4 ? 3 : 4)) gather_bp_kernel(const 
 #pragma unroll
                             for (int q = 1; q < L::NP; ++q)
                                 if (p == q) r = rows[2 * q + m];
-                            it[m].row = r && w0 != INT_MIN ? r + (size_t)view * vstride : nullptr;
-                            it[m].lw = lw ? lw + (size_t)view * d.nu : nullptr;
-                            it[m].w0 = w0 != INT_MIN ? w0 : 0;
+                            item(it[m], r, vi);
                         }
-                        stage_rows<true, MODE == kGatherPixel>(it, tab + (p * plane + vi * stride * L::kEntry) / 4, nullptr,
-                                                               A.win, d.nu, lane);
+                        stage_rows<true, MODE>(it, tab + (p * plane + vi * stride * kEntry) / 4, nullptr, A.win, d.nu,
+                                               lane);
                     }
                 } else {
                     for (int i = warp * 2; i < n; i += 16) {
                         RowItem<Tp> it[2];
 #pragma unroll
                         for (int m = 0; m < 2; ++m) {
-                            const int vi = min(i + m, n - 1), w0 = s_w0[qt + vi];
-                            const int view = vs + list[q0 + vi];
-                            it[m].row = rows[0] && w0 != INT_MIN ? rows[0] + (size_t)view * vstride : nullptr;
-                            it[m].lw = lw ? lw + (size_t)view * d.nu : nullptr;
-                            it[m].w0 = w0 != INT_MIN ? w0 : 0;
+                            item(it[m], rows[0], min(i + m, n - 1));
                         }
-                        float* t = tab + (size_t)i * stride * 2;
-                        stage_rows<false, MODE == kGatherPixel>(it, t, i + 1 < n ? t + stride * 2 : nullptr, A.win, d.nu,
-                                                                lane);
+                        float* t = tab + (size_t)i * stride * (kEntry / 4);
+                        stage_rows<false, MODE>(it, t, i + 1 < n ? t + stride * (kEntry / 4) : nullptr, A.win, d.nu, lane);
                     }
                 }
                 __syncthreads();
@@ -540,8 +604,38 @@ __global__ void __launch_bounds__(256, (S == 4 ? 3 : 4)) gather_bp_kernel(const 
                 const float py = (float)min(o == 0 ? xl_row : yl_row, g.ny - ty0 - 1);
                 for (int vi = 0; vi < n; ++vi) {
                     const float4 T = *reinterpret_cast<const float4*>(&s_tile[qt + vi]);  // jb, jx, jy, w
-                    const unsigned base = tab_addr + vi * stride * L::kEntry;
+                    const unsigned base = tab_addr + vi * stride * kEntry;
                     typename L::Point prev;
+                    // adjoint: the run's next edge, at x along the direction in which j moves
+                    // (dir: j itself or -j), in fractions f of a cell from its middle.  The
+                    // pixel before it takes its share of the last edge's cell, of this one's,
+                    // and the cells in between; no share, no term (0 x infinity).
+                    int cell_prev = 0;
+                    unsigned at_prev = 0;
+                    float x_prev = -INFINITY, f_prev = 0.f;
+                    auto edge = [&](int k, float x, float dir, auto fraction) {
+                        x = fmaxf(x, x_prev);  // (NaN: x_prev)
+                        const float tt = x + kMagic;
+                        const int cell = __float_as_int(tt), step = dir < 0.f ? -kEntry : kEntry;
+                        const unsigned at = base + kEntry * kMagicBits + (unsigned)(step * (cell - (int)kMagicBits));
+                        const float f = fraction(x - (tt - kMagic));
+                        const typename L::Point v = L::value(at, plane);
+                        if (k > 0) {
+                            const int n = cell - cell_prev;
+                            const float both = 0.5f * (f - f_prev);  // one cell: half from each of its readings
+                            const float a = n > 0 ? 0.5f - f_prev : both, b = n > 0 ? 0.5f + f : both;
+                            typename L::Point t = L::zero_point();
+                            if (!(a <= 0.f)) L::scale_add(t, prev, a);
+                            if (!(b <= 0.f)) L::scale_add(t, v, b);
+                            for (int i = 1; i < n; ++i) L::scale_add(t, L::value(at_prev + i * step, plane), 1.f);
+                            acc.add(k - 1, t);
+                        }
+                        prev = v;
+                        at_prev = at;
+                        cell_prev = cell;
+                        x_prev = x;
+                        f_prev = f;
+                    };
                     if constexpr (MODE == kGatherPixel) {
                         // 4 pixel centres; xs from the window's first cell's centre
                         float x, dx, cr = 0.f, dd = 1.f, dcr = 0.f, ddt = 0.f;
@@ -571,20 +665,29 @@ __global__ void __launch_bounds__(256, (S == 4 ? 3 : 4)) gather_bp_kernel(const 
                                 xs = fmaf((float)k, dx, x);
                             }
                             const float tt = __fadd_rd(xs, kMagic);  // floor
-                            acc.add(k, L::at(base + L::kEntry * __float_as_uint(tt), plane, xs - (tt - kMagic)), w);
+                            acc.add(k, L::at(base + kEntry * __float_as_uint(tt), plane, xs - (tt - kMagic)), w);
                         }
                     } else if constexpr (!FAN) {
                         // the run's first edge, half a pixel before its first centre
-                        const float e0 = fmaf(px - (o == 0 ? 0.5f : 0.f), T.y, fmaf(py - (o == 0 ? 0.f : 0.5f), T.z, T.x));
-                        const float step = o == 0 ? T.y : T.z;
+                        float e0 = fmaf(px - (o == 0 ? 0.5f : 0.f), T.y, fmaf(py - (o == 0 ? 0.f : 0.5f), T.z, T.x));
+                        float step = o == 0 ? T.y : T.z;
+                        const float dir = copysignf(1.f, step);
+                        if constexpr (MODE == kGatherAdjoint) {
+                            e0 *= dir;
+                            step *= dir;
+                        }
 #pragma unroll
                         for (int k = 0; k < 5; ++k) {
                             const float xs = fmaf((float)k, step, e0);
-                            const float tt = xs + kMagic;
-                            const typename L::Point p =
-                                L::at(base + L::kEntry * __float_as_uint(tt), plane, xs - (tt - kMagic));
-                            if (k > 0) acc.add(k - 1, prev, p, T.w);
-                            prev = p;
+                            if constexpr (MODE == kGatherAdjoint) {
+                                edge(k, xs, dir, [](float f) { return f; });
+                            } else {
+                                const float tt = xs + kMagic;
+                                const typename L::Point p =
+                                    L::at(base + kEntry * __float_as_uint(tt), plane, xs - (tt - kMagic));
+                                if (k > 0) acc.add(k - 1, prev, p, T.w);
+                                prev = p;
+                            }
                         }
                     } else {
                         const float4 B = *reinterpret_cast<const float4*>(&s_tile[qt + vi].bx);  // bx, by, gx, gy
@@ -606,10 +709,13 @@ __global__ void __launch_bounds__(256, (S == 4 ? 3 : 4)) gather_bp_kernel(const 
                             }
                         }
                         const float c3 = d.du * d.du * (2.f / 3.f);
-                        float jprev = 0.f, sgn = 0.f;
-                        // direction of j along the run
-                        if (MODE == kGatherAdjoint)
-                            sgn = T.w == T.w ? copysignf(1.f, idu * (o == 0 ? -(B.w + y0) : B.z + x0)) : T.w;
+                        // the adjoint takes j, du T and 1 / du along the direction of j
+                        const float dir = copysignf(1.f, idu * (o == 0 ? -(B.w + y0) : B.z + x0));
+                        const float jc = MODE == kGatherAdjoint ? dir * T.x : T.x;
+                        const float jdu = MODE == kGatherAdjoint ? dir * idu : idu;
+                        t0 *= dir;
+                        dt *= dir;
+                        float jprev = 0.f;
                         float crp = 0.f, dtp = 0.f;
 #pragma unroll
                         for (int k = 0; k < 5; ++k) {
@@ -618,23 +724,21 @@ __global__ void __launch_bounds__(256, (S == 4 ? 3 : 4)) gather_bp_kernel(const 
                             // atan(z) by its series (|z| <= 0.12: the next term is below 6e-10), unless a tile spans more
                             const float at = A.wide ? atanf(z)
                                                     : fmaf(z * z2, fmaf(z2, fmaf(z2, -1.f / 7.f, 0.2f), -1.f / 3.f), z);
-                            const float xs = fmaf(at, idu, T.x);
+                            const float xs = fmaf(at, jdu, jc);
+                            if constexpr (MODE == kGatherAdjoint) {
+                                const float duT = fmaf((float)k, dt, t0);
+                                edge(k, xs, dir, [&](float f) { return fmaf(fmaf(-f, f, 0.25f), fmaf(c3, f, duT), f); });
+                                continue;
+                            }
                             const float tt = xs + kMagic;
-                            float fr = xs - (tt - kMagic);
-                            if (MODE == kGatherAdjoint)
-                                fr = fmaf(fmaf(-fr, fr, 0.25f), fmaf(c3, fr, fmaf((float)k, dt, t0)), fr);
-                            const typename L::Point p = L::at(base + L::kEntry * __float_as_uint(tt), plane, fr);
+                            const typename L::Point p =
+                                L::at(base + kEntry * __float_as_uint(tt), plane, xs - (tt - kMagic));
                             if (k > 0) {
-                                float w;
-                                if (MODE == kGatherAdjoint) {
-                                    w = sgn;
-                                } else {
-                                    w = __fdividef(1.f, xs - jprev);
-                                    if (MODE == kGatherFbp) {
-                                        // dso^2 over the squared distance of the pixel's centre
-                                        const float cc = 0.5f * (cr + crp), dc = 0.5f * (dd + dtp);
-                                        w *= __fdividef(T.w, fmaf(cc, cc, dc * dc));
-                                    }
+                                float w = __fdividef(1.f, xs - jprev);
+                                if (MODE == kGatherFbp) {
+                                    // dso^2 over the squared distance of the pixel's centre
+                                    const float cc = 0.5f * (cr + crp), dc = 0.5f * (dd + dtp);
+                                    w *= __fdividef(T.w, fmaf(cc, cc, dc * dc));
                                 }
                                 acc.add(k - 1, prev, p, w);
                             }
@@ -781,9 +885,9 @@ int launch_gather(const GatherArgs& A, dim3 grid, int S, cudaStream_t s) {
         kern<<<grid, 256, smem, s>>>(A);
         return check_launch("gather_bp_kernel");
     };
-    if (S == 4) return go(gather_bp_kernel<FAN, MODE, 4, Tp>, gather_smem<4>(A.win));
-    if (S == 2) return go(gather_bp_kernel<FAN, MODE, 2, Tp>, gather_smem<2>(A.win));
-    return go(gather_bp_kernel<FAN, MODE, 1, Tp>, gather_smem<1>(A.win));
+    if (S == 4) return go(gather_bp_kernel<FAN, MODE, 4, Tp>, gather_smem<MODE, 4>(A.win));
+    if (S == 2) return go(gather_bp_kernel<FAN, MODE, 2, Tp>, gather_smem<MODE, 2>(A.win));
+    return go(gather_bp_kernel<FAN, MODE, 1, Tp>, gather_smem<MODE, 1>(A.win));
 }
 
 template <bool FAN, int MODE>
@@ -850,7 +954,9 @@ int gather_bp(void* img, const void* prj, const float* deg, const ctp_geometry& 
     if (mode == kGatherPixel)
         rc = geom == 1 ? launch_gather<false, kGatherPixel, float>(A, grid, S, s)
                        : launch_gather<true, kGatherPixel, float>(A, grid, S, s);
-    else if (geom == 1) rc = launch_gather_type<false, kGatherMean>(A, grid, S, flags, s);
+    else if (geom == 1)
+        rc = mode == kGatherAdjoint ? launch_gather_type<false, kGatherAdjoint>(A, grid, S, flags, s)
+                                    : launch_gather_type<false, kGatherMean>(A, grid, S, flags, s);
     else if (mode == kGatherMean) rc = launch_gather_type<true, kGatherMean>(A, grid, S, flags, s);
     else if (mode == kGatherFbp) rc = launch_gather_type<true, kGatherFbp>(A, grid, S, flags, s);
     else rc = launch_gather_type<true, kGatherAdjoint>(A, grid, S, flags, s);

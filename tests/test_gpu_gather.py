@@ -115,3 +115,50 @@ def test_pixel_driven(geom, nbatch, oracle):
         bad = np.abs(out.cpu().numpy() - ref) > 1e-4 * np.abs(ref).max()
         assert bad.sum() <= 2
         assert rel_l2(np.where(bad, ref, out.cpu().numpy()), ref) <= TOL
+
+
+@pytest.mark.parametrize("nbatch", [1, 2, 4])
+@pytest.mark.parametrize("geom", ["fan", "parallel"])
+def test_adjoint_keeps_cells_on_their_pixels(geom, nbatch, oracle):
+    """Exact adjoint: pixels outside a cell's footprint do not feel it, whether
+    it is not a number, infinite or six orders above the others."""
+    p = proj(geom, 70, 61, 96)
+    ang = angles(40, geom)
+    y = np.random.default_rng(5).uniform(0.5, 1, (nbatch, 40, 1, 96)).astype(np.float32)
+    cells = [(0, 3, 40), (nbatch - 1, 11, 50), (0, 29, 44), (nbatch - 1, 34, 52)]
+    mark = np.zeros_like(y)
+    for b, view, k in cells:
+        mark[b, view, 0, k] = 1
+    reach = oracle.dd_bp(p, mark, ang, geom, adjoint=True)
+    ref = oracle.dd_bp(p, np.where(mark > 0, 0, y).astype(np.float32), ang, geom, adjoint=True)
+    # an edge within rounding of the cell's may reach one pixel more: skip the fringe
+    fringe = np.zeros_like(reach, dtype=bool)
+    on = reach > 0
+    for dy in (-1, 0, 1):
+        for dx in (-1, 0, 1):
+            fringe |= np.roll(on, (dy, dx), (2, 3))
+    for bad in (np.nan, np.inf, 1e6):
+        x = np.where(mark > 0, np.float32(bad), y).astype(np.float32)
+        out = module(geom).distance_driven_bp(p, dev(x), dev(ang), adjoint=True).cpu().numpy()
+        away = ~fringe
+        assert np.isfinite(out[away]).all(), bad
+        assert np.abs(out - ref)[away].max() <= 4 * TOL * np.abs(ref).max(), bad
+        deep = reach > 0.05 * reach.max()
+        assert not np.isfinite(out[deep]).any() if not np.isfinite(bad) else (out[deep] > 1e3).all()
+        if bad == np.inf:
+            assert (out[deep] == np.inf).all()
+
+
+def test_fan_adjoint_at_its_widest_cells(oracle):
+    """Cells of 0.0098 rad, where the expansion in the cell's angle ends, on
+    tiles wide enough for the full arctangent."""
+    p = proj("fan", 40, 40, 81, pixel=6.0, cell=10.6)
+    check(p, angles(36, "fan"), "fan", oracle, 2, modes=("adjoint",))
+
+
+@pytest.mark.parametrize("geom", ["fan", "parallel"])
+def test_adjoint_of_fine_and_coarse_cells(geom, oracle):
+    """Cells from a fifth of a pixel (several within one) to six pixels."""
+    for factor, nu in ((0.2, 300), (6.0, 12)):
+        p = proj(geom, 37, 45, nu, cell=factor * (1.82 if geom == "fan" else 1.0))
+        check(p, angles(40, geom), geom, oracle, 3, modes=("adjoint",))
