@@ -207,6 +207,8 @@ __device__ __forceinline__ void stage_rows_per(const RowItem<Tp> (&it)[2], float
                 const int cell = it[m].w0 + k;
                 const float after = q + 1 < PER ? v[m][q + 1] : __shfl_down_sync(0xffffffffu, v[m][0], 1);
                 step[m] = cell >= 0 && cell + 1 < nu ? after - v[m][q] : 0.f;
+                // between an infinite cell and one that does not contradict it: infinite
+                if (isinf(v[m][q]) && (isfinite(after) || after == v[m][q])) step[m] = 0.f;
             }
             if (k > win) continue;
             if constexpr (PAIR) {

@@ -149,6 +149,27 @@ def test_adjoint_keeps_cells_on_their_pixels(geom, nbatch, oracle):
             assert (out[deep] == np.inf).all()
 
 
+@pytest.mark.parametrize("nbatch", [1, 3])
+@pytest.mark.parametrize("geom", ["fan", "parallel"])
+def test_pixel_driven_infinity(geom, nbatch, oracle):
+    """An infinite cell gives infinity, not NaN, between its neighbours' centres."""
+    p = proj(geom, 45, 38, 61)
+    ang = angles(50, geom)
+    y = np.random.default_rng(4).uniform(0, 1, (nbatch, 50, 1, 61)).astype(np.float32)
+    call, ref = ("fbp_bp", "fbp_bp") if geom == "fan" else ("pixel_driven_bp", "pixel_bp_parallel")
+    mark = np.zeros_like(y)
+    mark[0, 7, 0, 30] = mark[nbatch - 1, 20, 0, 25] = mark[nbatch - 1, 20, 0, 26] = 1
+    x = np.where(mark > 0, np.float32(np.inf), y)
+    reach = getattr(oracle, ref)(p, mark, ang)
+    out = getattr(module(geom), call)(p, dev(x), dev(ang)).cpu().numpy()
+    assert (out[reach > 1e-3 * reach.max()] == np.inf).all()
+    away = reach == 0
+    clean = getattr(oracle, ref)(p, np.where(mark > 0, 0, y).astype(np.float32), ang)
+    ok = away & np.isfinite(out)
+    assert away.sum() - ok.sum() <= 4  # a centre within rounding of the neighbour's
+    assert rel_l2(out[ok], clean[ok]) <= TOL
+
+
 def test_fan_adjoint_at_its_widest_cells(oracle):
     """Cells of 0.0098 rad, where the expansion in the cell's angle ends, on
     tiles wide enough for the full arctangent."""
