@@ -472,7 +472,8 @@ constexpr int kBpGroup = 8;    // z cells per group (skipped when no ray of the 
 constexpr int kBpWin = 64;     // detector columns of a staged window (a row spans all banks twice)
 constexpr int kBpRows = 64;    // rows of a staged window: kBpRows + 1 running sums per column
 constexpr int kBpStep = 2;     // views staged and taken between two barriers
-constexpr int kBpViews = 32;   // views whose constants are computed together
+constexpr int kBpViews = 20;   // views whose constants are computed together (at most a warp's lanes)
+constexpr int kBpTerm = 60;    // views added up in registers before the sums join the volume (whole kBpViews)
 // dynamic shared memory of a block, in floats: two buffers of staged windows,
 // and the split rows' sums, one per plane and thread
 constexpr int kBpWindow = (kBpRows + 1) * kBpWin;
@@ -497,6 +498,14 @@ struct BpView {
     int row, nrow;                  // first running sum used, and how many
     int g0, g1;                     // groups of z cells that rays reach, [g0, g1)
     int vi;                         // view within the launch's views
+};
+
+// The x-y line of a detector column over one tile: alpha (relative to ar) of its
+// first x and y planes and per pixel, in FP32; and in FP64 the difference between
+// the lower x and the lower y plane of the tile's first pixel, and its steps.
+struct BpLine {
+    float x0, dx, y0, dy;
+    double e, ex, ey;
 };
 
 __device__ __forceinline__ void cp_async16(float* dst, const float* src) {
@@ -619,13 +628,18 @@ __global__ void __launch_bounds__(128) bp_fit_kernel(UprightView* __restrict__ v
 //   voxel's sum is the difference between its two planes, times aB - aA.
 // So a voxel costs one table read per crossing line, whatever the number of
 // rows that meet it, and nothing is scattered.  Alphas are relative to the
-// tile's centre, from per-line coefficients rounded from FP64, which keeps the
-// chords' rounding at 1e-6 of a voxel.
+// tile's centre, from per-line coefficients rounded from FP64.  A chord is a
+// difference of two of them, so it is taken from the FP64 distance between the
+// pixel's x and y planes instead (two multiply-adds per pixel and line), and the
+// sums of kBpTerm views at a time join the volume.  64 x 192 x 192 voxels, 180
+// views: 4.64e-7 from 64 bits (ray by ray 4.64e-7; with chords of FP32 alphas,
+// 1e-6 of a voxel each, 4.9e-7, and with one sum over the views besides 5.15e-7),
+// for 8% of the time.
 //
 // Bound by issue: per plane and crossing line two saturating multiply-adds, two
 // directed roundings, a compare and a read.  The same volume and views: 14.9 ms
-// ray by ray (siddon_bp_kernel's atomics), 5.96 ms here; 33 x 187 x 201 voxels,
-// 97 views of 251 x 37 cells: 362 -> 330 us with the set-up launches.  Measured
+// ray by ray (siddon_bp_kernel's atomics), 6.45 ms here; 33 x 187 x 201 voxels,
+// 97 views of 251 x 37 cells: 362 -> 350 us with the set-up launches.  Measured
 // and not taken, same volume: columns as the rows of the staged window (bank
 // conflicts) 6.74 ms; one view between barriers 6.10; three blocks per SM at 80
 // registers 6.56; two threads per pixel, every other line each, 9.2.
@@ -638,7 +652,7 @@ __global__ void __launch_bounds__(256, 2) columns_bp_kernel(float* __restrict__ 
     extern __shared__ float4 s_raw[];
     float* s_P = reinterpret_cast<float*>(s_raw);     // [2][kBpStep][kBpRows + 1][kBpWin]
     float* s_split = s_P + kBpStageFloats;            // [kBpZ + 1][256] sums of the split rows, per plane and thread
-    __shared__ float4 s_line[2][kBpStep][kBpWin];
+    __shared__ BpLine s_line[2][kBpStep][kBpWin];
     __shared__ float2 s_rowz[2][kBpStep][kBpRows + 1];  // staged rows' z at alpha ar from the first plane, see row_z
     __shared__ BpView s_view[kBpViews];
     __shared__ int s_n;
@@ -650,6 +664,7 @@ __global__ void __launch_bounds__(256, 2) columns_bp_kernel(float* __restrict__ 
     const int z0 = zc * zper, nz = min(zper, g.nz - z0);
     const int tx = tid & (kBpTile - 1), ty = tid / kBpTile;
     const float kx = (float)tx, ky = (float)ty;
+    const double dkx = tx, dky = ty;
     const float* Pb = P + (size_t)b * nviews * (d.nv + 1) * pitch;
 
     float acc[kBpZ];
@@ -662,21 +677,28 @@ __global__ void __launch_bounds__(256, 2) columns_bp_kernel(float* __restrict__ 
     // of its own pixel for every alpha, and of no other.
     auto line = [&](const BpView& V, int c) {
         const double2 q = inv[(size_t)V.vi * d.nu + V.first + c];
-        float4 L = make_float4((float)(V.bx * q.x - (double)V.ar), (float)q.x, (float)(V.by * q.y - (double)V.ar),
-                               (float)q.y);
+        double x0 = V.bx * q.x - (double)V.ar, dx = q.x, y0 = V.by * q.y - (double)V.ar, dy = q.y;
         if (isinf(q.x) || isinf(q.y)) {
             const UprightView& w = views[view0 + V.vi];
             const int iu = V.first + c;
             const double a = V.ar;
             if (isinf(q.x)) {
-                L.y = 1024.f;
-                L.x = -1024.f * (float)((int)floor(w.sx + a * (w.dx0 + iu * w.ux)) - tx0) - 512.f;
+                dx = 1024.0;
+                x0 = -1024.0 * ((int)floor(w.sx + a * (w.dx0 + iu * w.ux)) - tx0) - 512.0;
             }
             if (isinf(q.y)) {
-                L.w = 1024.f;
-                L.z = -1024.f * (float)((int)floor(w.sy + a * (w.dy0 + iu * w.uy)) - ty0) - 512.f;
+                dy = 1024.0;
+                y0 = -1024.0 * ((int)floor(w.sy + a * (w.dy0 + iu * w.uy)) - ty0) - 512.0;
             }
         }
+        BpLine L;
+        L.x0 = (float)x0;
+        L.dx = (float)dx;
+        L.y0 = (float)y0;
+        L.dy = (float)dy;
+        L.e = (x0 + fmin(dx, 0.0)) - (y0 + fmin(dy, 0.0));
+        L.ex = dx;
+        L.ey = dy;
         return L;
     };
 
@@ -716,15 +738,17 @@ __global__ void __launch_bounds__(256, 2) columns_bp_kernel(float* __restrict__ 
     // two, which rounds alike).
     const float frows = (float)rows, irows = 1.f / frows;
     auto column = [&](const BpView& V, int buf, int j, int c) {
-        const float4 L = s_line[buf][j][c];
+        const BpLine& L = s_line[buf][j][c];
         const float* col = s_P + (buf * kBpStep + j) * kBpWindow + c;
-        const float ax0 = fmaf(kx, L.y, L.x), ax1 = fmaf(kx + 1.f, L.y, L.x);
-        const float ay0 = fmaf(ky, L.w, L.z), ay1 = fmaf(ky + 1.f, L.w, L.z);
-        const float lo = fmaxf(fminf(ax0, ax1), fminf(ay0, ay1));
-        const float hi = fminf(fmaxf(ax0, ax1), fmaxf(ay0, ay1));
-        if (!(hi > lo)) return;
-        const float da = (hi - lo) * V.sgn;
-        const float aA = V.ar + lo, aB = V.ar + hi;
+        // from the lower x plane to the lower y plane, and the chord: the pixel's
+        // extent along the axis that it spans, less what the other plane cuts off
+        const float e = (float)fma(dkx, L.ex, fma(-dky, L.ey, L.e));
+        const float wx = fabsf(L.dx), wy = fabsf(L.dy);
+        const float chord = fminf(fminf(wx, wy), fminf(wx + e, wy - e));
+        if (!(chord > 0.f)) return;
+        const float lo = e < 0.f ? fmaf(ky, L.dy, L.y0) + fminf(L.dy, 0.f) : fmaf(kx, L.dx, L.x0) + fminf(L.dx, 0.f);
+        const float da = chord * V.sgn;
+        const float aA = V.ar + lo, aB = V.ar + (lo + chord);
         const float gA = __fdividef(V.ikv, aA), gB = __fdividef(V.ikv, aB);
         const int g0 = V.g0, g1 = V.g1;
         const float zz0 = V.zz0, vc = V.vc, kbf = V.kbf, kvf = V.kvf;
@@ -773,7 +797,7 @@ __global__ void __launch_bounds__(256, 2) columns_bp_kernel(float* __restrict__ 
                 const float2 rz = s_rowz[buf][j][k];
                 const float kappa = fmaf((float)k, kvf, kbf);
                 const float f = __saturatef(__fdividef(fmaf(-lo, kappa, (float)(q - __float_as_int(rz.x)) - rz.y),
-                                                       (hi - lo) * kappa));
+                                                       chord * kappa));
                 part = fmaf(col[(k + 1) * kBpWin] - col[k * kBpWin], kA > kB ? f - 1.f : 1.f - f, part);
             }
             s_split[q * 256 + tid] += part * da;
@@ -803,13 +827,39 @@ __global__ void __launch_bounds__(256, 2) columns_bp_kernel(float* __restrict__ 
         }
     };
 
+    // the sums so far join the volume
+    auto store = [&]() {
+        int ix = tx0 + tx;
+        asm volatile("" : "+r"(ix));  // (its addresses are formed here, not kept through the views)
+        const int iy = ty0 + ty;
+        const bool in = ix < g.nx && iy < g.ny;
+        float* o = img + (((size_t)b * g.nz + z0) * g.ny + iy) * g.nx + ix;
+        float below = s_split[tid];
+#pragma unroll
+        for (int q = 0; q < kBpZ; ++q) {
+            const float above = s_split[(q + 1) * 256 + tid], sum = acc[q] + (above - below);
+            if (in && q < nz) {
+                if (ATOMIC)
+                    atomicAdd(o, sum);
+                else
+                    *o += sum;
+            }
+            o += (size_t)g.nx * g.ny;
+            s_split[q * 256 + tid] = 0.f;
+            acc[q] = 0.f;
+            below = above;
+        }
+        s_split[kBpZ * 256 + tid] = 0.f;
+    };
+
     const int vb = part * vper, ve = min(nviews, vb + vper);
     for (int v0 = vb; v0 < ve; v0 += kBpViews) {
+        if (v0 > vb && (v0 - vb) % kBpTerm == 0) store();
         __syncthreads();
         if (tid < 32) {
             const int vi = v0 + tid;
             BpView V;
-            bool use = vi < ve && views[view0 + vi].upright;
+            bool use = tid < kBpViews && vi < ve && views[view0 + vi].upright;
             if (use) use = bp_view(views[view0 + vi], tx0, ty0, z0, nz, g, d, V);
             V.c1 = min(V.c1, kBpWin);  // (bp_fit_kernel)
             V.vi = vi;
@@ -827,19 +877,7 @@ __global__ void __launch_bounds__(256, 2) columns_bp_kernel(float* __restrict__ 
             compute(i, n, buf);
         }
     }
-    const int ix = tx0 + tx, iy = ty0 + ty;
-    if (ix >= g.nx || iy >= g.ny) return;
-    float* o = img + (((size_t)b * g.nz + z0) * g.ny + iy) * g.nx + ix;
-    const size_t plane_px = (size_t)g.nx * g.ny;
-#pragma unroll
-    for (int q = 0; q < kBpZ; ++q) {
-        if (q >= nz) break;
-        const float sum = acc[q] + (s_split[(q + 1) * 256 + tid] - s_split[q * 256 + tid]);
-        if (ATOMIC)
-            atomicAdd(o + q * plane_px, sum);
-        else
-            o[q * plane_px] += sum;
-    }
+    store();
 }
 
 // Bytes of running sums held at a time: the views are taken in groups.
@@ -1015,14 +1053,13 @@ int columns_bp(ColumnsPlan& plan, char* scratch, float* img, const void* prj, co
             for (int p = 2; p <= std::min(16, n / 8); ++p)
                 if (rounds(p) < 0.97 * rounds(parts)) parts = p;
         }
-        const int vper = (n + parts - 1) / parts;
         const dim3 grid((unsigned)tiles, (unsigned)(zchunks * parts), (unsigned)g.nbatch);
         int rows = 8;  // rows staged: a power of two (see column), nv or more up to kBpRows
         while (rows < kBpRows && rows < (int)g.nv) rows *= 2;
         auto k = parts > 1 ? columns_bp_kernel<true> : columns_bp_kernel<false>;
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k<<<grid, 256, smem, s>>>(img, P, inv, plan.views, (int)v0, n, vper, gr, dt, (int)bp_pitch(g), rows, zper,
-                                  zchunks);
+        k<<<grid, 256, smem, s>>>(img, P, inv, plan.views, (int)v0, n, (n + parts - 1) / parts, gr, dt, (int)bp_pitch(g),
+                                  rows, zper, zchunks);
         if ((rc = check_launch("columns_bp_kernel"))) return rc;
     }
     return CTP_OK;
