@@ -200,24 +200,40 @@ __device__ __forceinline__ void stage_rows_per(const RowItem<Tp> (&it)[2], float
             }
         }
     } else if constexpr (MODE == kGatherPixel) {
+        const float next[2] = {__shfl_down_sync(0xffffffffu, v[0][0], 1), __shfl_down_sync(0xffffffffu, v[1][0], 1)};
+        auto step_of = [&](int m, int q, float& after) {
+            const int cell = it[m].w0 + k0 + q;
+            after = q + 1 < PER ? v[m][q + 1] : next[m];
+            return cell >= 0 && cell + 1 < nu ? after - v[m][q] : 0.f;
+        };
+        auto put = [&](int q, float s0, float s1) {
+            const int k = k0 + q;
+            if (k > win) return;
+            if constexpr (PAIR) {
+                reinterpret_cast<float4*>(t0)[k] = make_float4(v[0][q], v[1][q], s0, s1);
+            } else {
+                reinterpret_cast<float2*>(t0)[k] = make_float2(v[0][q], s0);
+                if (t1) reinterpret_cast<float2*>(t1)[k] = make_float2(v[1][q], s1);
+            }
+        };
+        float finite = 0.f, after;  // NaN when a step is not finite
 #pragma unroll
         for (int q = 0; q < PER; ++q) {
-            const int k = k0 + q;
-            float step[2];
+            const float s0 = step_of(0, q, after), s1 = step_of(1, q, after);
+            finite = fmaf(s0, 0.f, fmaf(s1, 0.f, finite));
+            put(q, s0, s1);
+        }
+        if (finite != 0.f) {
+            // from an infinite cell to one that does not contradict it: no step
 #pragma unroll
-            for (int m = 0; m < 2; ++m) {
-                const int cell = it[m].w0 + k;
-                const float after = q + 1 < PER ? v[m][q + 1] : __shfl_down_sync(0xffffffffu, v[m][0], 1);
-                step[m] = cell >= 0 && cell + 1 < nu ? after - v[m][q] : 0.f;
-                // between an infinite cell and one that does not contradict it: infinite
-                if (!isfinite(step[m]) && isinf(v[m][q]) && (isfinite(after) || after == v[m][q])) step[m] = 0.f;
-            }
-            if (k > win) continue;
-            if constexpr (PAIR) {
-                reinterpret_cast<float4*>(t0)[k] = make_float4(v[0][q], v[1][q], step[0], step[1]);
-            } else {
-                reinterpret_cast<float2*>(t0)[k] = make_float2(v[0][q], step[0]);
-                if (t1) reinterpret_cast<float2*>(t1)[k] = make_float2(v[1][q], step[1]);
+            for (int q = 0; q < PER; ++q) {
+                float s[2];
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    s[m] = step_of(m, q, after);
+                    if (isinf(v[m][q]) && (isfinite(after) || after == v[m][q])) s[m] = 0.f;
+                }
+                put(q, s[0], s[1]);
             }
         }
     } else {
