@@ -24,6 +24,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "siddon_columns.cuh"
 
@@ -415,55 +416,127 @@ __global__ void __launch_bounds__(256, 5) columns_fp_kernel(Tout* __restrict__ p
 // ---------------------------------------------------------------------------
 // Back projection.
 
-// Running sums over the rows of every detector column of the upright views,
-// each cell times its ray's length: P[b][view][k][iu] = sum over v < k, k = 0
-// .. nv, in FP64, stored FP32 (row pitch a multiple of 4 cells); and per column
-// the reciprocal steps of its x-y line.  A view that holds an infinity or NaN
-// is listed for the ray-driven kernel (running sums would spread it over the
-// column).
-template <typename Tin>
-__global__ void __launch_bounds__(128) columns_prefix_kernel(float* __restrict__ P, double2* __restrict__ inv,
-                                                             const Tin* __restrict__ prj,
-                                                             const UprightView* __restrict__ views,
-                                                             int* __restrict__ bad, int nview, int view0, int nviews,
-                                                             Grid g, Det d, int pitch) {
-    const int iu = blockIdx.x * 128 + threadIdx.x;
-    const int vi = blockIdx.y, b = blockIdx.z;
-    const int view = view0 + vi;
-    if (iu >= d.nu || !views[view].upright) return;
-    const UprightView& w = views[view];
-    if (b == 0) {
-        // steps below 1e-6 voxels over the whole ray count as none (siddon.cu
-        // kEps): marked by an infinite reciprocal
-        const double dx = w.dx0 + iu * w.ux, dy = w.dy0 + iu * w.uy;
-        inv[(size_t)vi * d.nu + iu] = make_double2(fabs(dx) < 1e-6 ? INFINITY : 1.0 / dx,
-                                                   fabs(dy) < 1e-6 ? INFINITY : 1.0 / dy);
-    }
-    const float l2 = (float)xy_length2(w, iu, g);
-    const float k0 = (float)(w.k0 * g.dz), kv = (float)(w.kv * g.dz);
-    const Tin* src = prj + (((size_t)b * nview + view) * d.nv) * d.nu + iu;
-    float* out = P + (((size_t)b * nviews + vi) * (d.nv + 1)) * pitch + iu;
-    out[0] = 0.f;
-    double run = 0.0;
-    float top = 0.f;
-#pragma unroll 8
-    for (int v = 0; v < d.nv; ++v) {
-        const float z = fmaf((float)v, kv, k0);
-        run += (double)(ldf(src + (size_t)v * d.nu) * sqrtf(fmaf(z, z, l2)));
-        top = fmaxf(top, fabsf((float)run));
-        out[(size_t)(v + 1) * pitch] = (float)run;
-    }
-    if (!isfinite((float)run) || isinf(top)) bad[vi] = 1;
+// Running sums of the detector columns restart every kSumStep rows and run over
+// kSumRows of them, so that any kBpRows + 1 of them in a row lie within one run
+// and no sum holds more than kSumRows cells, however tall the detector.
+constexpr int kSumStep = 32;
+constexpr int kSumRows = 96;
+__host__ __device__ __forceinline__ int sum_runs(int nv) {
+    return nv <= kSumRows ? 1 : (nv - kSumRows + kSumStep - 1) / kSumStep + 1;
+}
+// Rows of sums of one view: the runs one after the other, kSumRows + 1 each.
+__host__ __device__ __forceinline__ int sum_rows(int nv) {
+    return nv <= kSumRows ? nv + 1 : sum_runs(nv) * (kSumRows + 1);
 }
 
-// Views whose running sums are not finite go to the ray-driven list instead.
-__global__ void retire_views_kernel(UprightView* __restrict__ views, int* __restrict__ rest,
-                                    const int* __restrict__ bad, int view0, int nviews) {
-    for (int vi = threadIdx.x; vi < nviews; vi += blockDim.x)
-        if (bad[vi]) {
+// Running sums over the rows of every detector column of the upright views,
+// each cell times its ray's length: P[b][view][run][k][iu] = sum over the run's
+// first k cells, in FP64, stored FP32 (row pitch a multiple of 4 cells); and per
+// column the reciprocal steps of its x-y line.  stats[b][view][run][block]: the
+// sum of the cells' magnitudes (each cell once) and the largest sum's, infinite
+// when a cell is not finite; zeros for views that are not upright.
+template <typename Tin>
+__global__ void __launch_bounds__(128) columns_prefix_kernel(float* __restrict__ P, double2* __restrict__ inv,
+                                                             float2* __restrict__ stats, const Tin* __restrict__ prj,
+                                                             const UprightView* __restrict__ views, int nview, int view0,
+                                                             int nviews, Grid g, Det d, int pitch) {
+    __shared__ float2 s_stat[4];
+    const int iu = blockIdx.x * 128 + threadIdx.x;
+    const int runs = sum_runs(d.nv), vi = blockIdx.y, run_i = blockIdx.z % runs, b = blockIdx.z / runs;
+    const int view = view0 + vi;
+    float mag = 0.f, top = 0.f;
+    if (iu < d.nu && views[view].upright) {
+        const UprightView& w = views[view];
+        if (blockIdx.z == 0) {
+            // steps below 1e-6 voxels over the whole ray count as none (siddon.cu
+            // kEps): marked by an infinite reciprocal
+            const double dx = w.dx0 + iu * w.ux, dy = w.dy0 + iu * w.uy;
+            inv[(size_t)vi * d.nu + iu] = make_double2(fabs(dx) < 1e-6 ? INFINITY : 1.0 / dx,
+                                                       fabs(dy) < 1e-6 ? INFINITY : 1.0 / dy);
+        }
+        const float l2 = (float)xy_length2(w, iu, g);
+        const float k0 = (float)(w.k0 * g.dz), kv = (float)(w.kv * g.dz);
+        const int va = run_i * kSumStep, rows = min(kSumRows, d.nv - va);
+        const int own = run_i + 1 < runs ? kSumStep : rows;  // rows that the next run does not start in
+        const Tin* src = prj + (((size_t)b * nview + view) * d.nv + va) * d.nu + iu;
+        float* out = P + (((size_t)b * nviews + vi) * sum_rows(d.nv) + run_i * (kSumRows + 1)) * pitch + iu;
+        out[0] = 0.f;
+        double run = 0.0;
+#pragma unroll 8
+        for (int v = 0; v < rows; ++v) {
+            const float z = fmaf((float)(va + v), kv, k0);
+            const float p = ldf(src + (size_t)v * d.nu) * sqrtf(fmaf(z, z, l2));
+            run += (double)p;
+            if (v < own) mag += fabsf(p);
+            top = fmaxf(top, fabsf((float)run));
+            out[(size_t)(v + 1) * pitch] = (float)run;
+        }
+        if (!isfinite((float)run) || isinf(top)) top = INFINITY;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        mag += __shfl_xor_sync(0xffffffffu, mag, o);
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    }
+    if ((threadIdx.x & 31) == 0) s_stat[threadIdx.x >> 5] = make_float2(mag, top);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < 4; ++k) {
+            mag += s_stat[k].x;
+            top = fmaxf(top, s_stat[k].y);
+        }
+        stats[(((size_t)b * nviews + vi) * runs + run_i) * gridDim.x + blockIdx.x] = make_float2(mag, top);
+    }
+}
+
+// Views that the running sums do not serve go to the ray-driven list instead: a
+// sum that is not finite would spread over the column, and one far above the
+// other cells would cost them their bits.  A voxel's sum is a difference of two
+// FP32 numbers of the largest sum's size, so it may be off by 2^-24 of that in
+// one view; kOutlier times the cells of a run at their mean magnitude (over the
+// views at hand) bounds this to 2^-24 x 32 x 96 = 2e-4 of a mean cell a view,
+// 4e-7 of a voxel that 360 views meet with a cell or two each.  Sums reach
+// one over the share of the columns that the object covers: 3% stay.
+// One block; sums in a fixed order.
+constexpr float kOutlier = 32.f;
+__global__ void __launch_bounds__(256) retire_views_kernel(UprightView* __restrict__ views, int* __restrict__ rest,
+                                                           const float2* __restrict__ stats, int view0, int nviews,
+                                                           int nbatch, int per_view, Det d) {
+    __shared__ float s_mag[256];
+    __shared__ int s_up[256];
+    float mag = 0.f;
+    int up = 0;
+    for (int vi = threadIdx.x; vi < nviews; vi += blockDim.x) {
+        if (!views[view0 + vi].upright) continue;
+        ++up;
+        for (int b = 0; b < nbatch; ++b)
+            for (int k = 0; k < per_view; ++k) {
+                const float2 t = stats[((size_t)b * nviews + vi) * per_view + k];
+                if (isfinite(t.y)) mag += t.x;
+            }
+    }
+    s_mag[threadIdx.x] = mag;
+    s_up[threadIdx.x] = up;
+    __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+        if (threadIdx.x < o) {
+            s_mag[threadIdx.x] += s_mag[threadIdx.x + o];
+            s_up[threadIdx.x] += s_up[threadIdx.x + o];
+        }
+        __syncthreads();
+    }
+    const float mean = s_mag[0] / ((float)max(s_up[0], 1) * (float)nbatch * (float)d.nu * (float)d.nv);
+    const float most = kOutlier * (float)min(d.nv, kSumRows) * mean;
+    for (int vi = threadIdx.x; vi < nviews; vi += blockDim.x) {
+        if (!views[view0 + vi].upright) continue;
+        bool keep = true;
+        for (int b = 0; b < nbatch; ++b)
+            for (int k = 0; k < per_view; ++k) keep = keep && stats[((size_t)b * nviews + vi) * per_view + k].y <= most;
+        if (!keep) {
             views[view0 + vi].upright = 0;
             rest[1 + atomicAdd(rest, 1)] = view0 + vi;
         }
+    }
 }
 
 constexpr int kBpTile = 16;    // pixel columns per side of a block's tile
@@ -665,7 +738,7 @@ __global__ void __launch_bounds__(256, 2) columns_bp_kernel(float* __restrict__ 
     const int tx = tid & (kBpTile - 1), ty = tid / kBpTile;
     const float kx = (float)tx, ky = (float)ty;
     const double dkx = tx, dky = ty;
-    const float* Pb = P + (size_t)b * nviews * (d.nv + 1) * pitch;
+    const float* Pb = P + (size_t)b * nviews * sum_rows(d.nv) * pitch;
 
     float acc[kBpZ];
 #pragma unroll
@@ -718,11 +791,13 @@ __global__ void __launch_bounds__(256, 2) columns_bp_kernel(float* __restrict__ 
             if (i + j >= n) break;
             const BpView& V = s_view[i + j];
             float* dst = s_P + (buf * kBpStep + j) * kBpWindow + 4 * half;
-            const float* src = Pb + (size_t)V.vi * (d.nv + 1) * pitch + V.first + 4 * half;
-            const int row = V.row, c1 = V.c1;
+            // the run of sums that the rows lie in
+            const int run = min(V.row / kSumStep, sum_runs(d.nv) - 1), va = run * kSumStep;
+            const float* src = Pb + ((size_t)V.vi * sum_rows(d.nv) + run * (kSumRows + 1)) * pitch + V.first + 4 * half;
+            const int row = V.row - va, last = min(kSumRows, d.nv - va), c1 = V.c1;
             if (4 * half < c1)
                 for (int r = 2 * (tid >> 5) + (lane >> 4); r <= rows; r += 16)
-                    cp_async16(dst + r * kBpWin, src + (size_t)min(row + r, d.nv) * pitch);
+                    cp_async16(dst + r * kBpWin, src + (size_t)min(row + r, last) * pitch);
             const int c = tid - j * 64;  // (warps 0, 1 and 2, 3; rows: 4, 5 and 6, 7)
             if (c >= 0 && c < c1) s_line[buf][j][c] = line(V, c);
             const int k = tid - 128 - j * 64;
@@ -972,7 +1047,10 @@ namespace {
 
 size_t bp_pitch(const ctp_geometry& g) { return (g.nu + 3) & ~(size_t)3; }
 
-size_t bp_view_bytes(const ctp_geometry& g) { return g.nbatch * (g.nv + 1) * bp_pitch(g) * sizeof(float); }
+size_t bp_view_bytes(const ctp_geometry& g) { return g.nbatch * sum_rows((int)g.nv) * bp_pitch(g) * sizeof(float); }
+
+// Statistics of a view (columns_prefix_kernel), per batch item.
+size_t bp_view_stats(const ctp_geometry& g) { return sum_runs((int)g.nv) * ((g.nu + 127) / 128); }
 
 size_t bp_views(const ctp_geometry& g) {
     return std::max<size_t>(1, std::min<size_t>(g.nview, kPrefixBytes / bp_view_bytes(g)));
@@ -994,14 +1072,14 @@ bool columns_bp_applies(const ctp_geometry& g, unsigned flags) {
     const double ray = lines * g.nv / 0.58e9;
     const double column = lines * 1.27 * (40.0 * ((g.nz + kBpZ - 1) / kBpZ) + 10.0 * g.nz) / 2.14e10;
     if (!(flags & CTP_FLAG_SIDDON_COLUMNS) && ray < 1.75 * column + 0.06) return false;
-    return g.nz >= 4 && g.nv >= 2 && g.nbatch <= 65535 && g.nview <= 65535 && bp_view_bytes(g) <= kPrefixBytes &&
-           g.nu < (1u << 28);
+    return g.nz >= 4 && g.nv >= 2 && g.nv < (1u << 28) && g.nbatch * sum_runs((int)g.nv) <= 65535 &&
+           g.nview <= 65535 && bp_view_bytes(g) <= kPrefixBytes && g.nu < (1u << 28);
 }
 
 size_t columns_bp_bytes(const ctp_geometry& g) {
     const size_t nv = bp_views(g);
     return setup_bytes(g) + align_up(nv * bp_view_bytes(g)) + align_up(nv * g.nu * sizeof(double2)) +
-           align_up(nv * sizeof(int));
+           align_up(nv * g.nbatch * bp_view_stats(g) * sizeof(float2));
 }
 
 int columns_bp(ColumnsPlan& plan, char* scratch, float* img, const void* prj, const float* dc, const float* du_,
@@ -1014,7 +1092,7 @@ int columns_bp(ColumnsPlan& plan, char* scratch, float* img, const void* prj, co
     p += align_up(nv * bp_view_bytes(g));
     double2* inv = reinterpret_cast<double2*>(p);
     p += align_up(nv * g.nu * sizeof(double2));
-    int* bad = reinterpret_cast<int*>(p);
+    float2* stats = reinterpret_cast<float2*>(p);
     int sms = 148, dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int zchunks = (int)((g.nz + kBpZ - 1) / kBpZ);
@@ -1028,20 +1106,18 @@ int columns_bp(ColumnsPlan& plan, char* scratch, float* img, const void* prj, co
     if ((rc = check_launch("bp_fit_kernel"))) return rc;
     for (size_t v0 = 0; v0 < g.nview; v0 += nv) {
         const int n = (int)std::min(nv, g.nview - v0);
-        cudaError_t e = cudaMemsetAsync(bad, 0, n * sizeof(int), s);
-        if (e != cudaSuccess) return set_error((int)e, "siddon_bp memset: %s", cudaGetErrorString(e));
-        const dim3 pg((unsigned)((g.nu + 127) / 128), (unsigned)n, (unsigned)g.nbatch);
-        if (flags & CTP_FLAG_IN_BF16)
-            columns_prefix_kernel<__nv_bfloat16><<<pg, 128, 0, s>>>(P, inv, (const __nv_bfloat16*)prj, plan.views, bad,
-                                                                    (int)g.nview, (int)v0, n, gr, dt, (int)bp_pitch(g));
-        else if (flags & CTP_FLAG_IN_FP16)
-            columns_prefix_kernel<__half><<<pg, 128, 0, s>>>(P, inv, (const __half*)prj, plan.views, bad, (int)g.nview,
-                                                             (int)v0, n, gr, dt, (int)bp_pitch(g));
-        else
-            columns_prefix_kernel<float><<<pg, 128, 0, s>>>(P, inv, (const float*)prj, plan.views, bad, (int)g.nview,
-                                                            (int)v0, n, gr, dt, (int)bp_pitch(g));
+        const dim3 pg((unsigned)((g.nu + 127) / 128), (unsigned)n, (unsigned)(g.nbatch * sum_runs((int)g.nv)));
+        auto prefix = [&](auto* in) {
+            using Tin = std::remove_pointer_t<decltype(in)>;
+            columns_prefix_kernel<Tin><<<pg, 128, 0, s>>>(P, inv, stats, (const Tin*)prj, plan.views, (int)g.nview,
+                                                          (int)v0, n, gr, dt, (int)bp_pitch(g));
+        };
+        if (flags & CTP_FLAG_IN_BF16) prefix((__nv_bfloat16*)nullptr);
+        else if (flags & CTP_FLAG_IN_FP16) prefix((__half*)nullptr);
+        else prefix((float*)nullptr);
         if ((rc = check_launch("columns_prefix_kernel"))) return rc;
-        retire_views_kernel<<<1, 256, 0, s>>>(plan.views, plan.rest, bad, (int)v0, n);
+        retire_views_kernel<<<1, 256, 0, s>>>(plan.views, plan.rest, stats, (int)v0, n, (int)g.nbatch,
+                                               (int)bp_view_stats(g), dt);
         if ((rc = check_launch("retire_views_kernel"))) return rc;
         // launches of few waves (two blocks per SM) split the views into the
         // parts, added with atomics, that take the fewest rounds of views; a part
