@@ -6,17 +6,16 @@
 // distanceDriven3DUtils.cu:10-31, ProjectConeToDetCart :45-56, and the 2D box
 // integral IntegralBoxXY cudaMath.cu:336-404.
 //
-// Forward: one thread per ray; per z plane the normalised integral of the
-// plane over the footprint rectangle of the cell.  Back projection
-// (reference-parity form): one thread per voxel; per view the normalised
-// integral of the length-weighted projection over the voxel's projected
-// rectangle.  The per-cell ray-length weight is applied once in a pre-pass
-// into the workspace.  The rectangles' two sides are separable, so threads
-// share the work along y: 64 x 256 x 512 voxels, 25 views of 1024 x 512 cells of
-// 0.25 mm, forward and back 4.55 -> 1.58 ms against one rectangle per thread and
-// plane (or view); both kernels are bound by instruction issue and the L1.
-// Cells much finer or coarser than the pixels keep one rectangle per thread
-// (shared_rows).
+// Forward: per ray and z plane the normalised integral of the plane over the
+// footprint rectangle of the cell.  Back projection (reference-parity form): per
+// voxel and view the normalised integral of the length-weighted projection over
+// the voxel's projected rectangle.  The per-cell ray-length weight is applied
+// once in a pre-pass into the workspace.  The rectangles' two sides are
+// separable, so a thread takes 8 to 32 rays (voxels) of one column and shares
+// the work along y: 64 x 256 x 512 voxels, 25 views of 1024 x 512 cells of 0.25 mm,
+// forward and back 4.55 -> 1.63 ms against one rectangle per thread and plane (or
+// view); both kernels are bound by instruction issue and the L1.  Cells much
+// finer or coarser than the pixels keep one rectangle per thread (shared_rows).
 // Unlike the reference, every batch item reads its own weighted projections
 // (the reference reads item 0's for all items, distanceDriven3DBoxInt.cu:257-259).
 #include <cuda_runtime.h>
@@ -485,15 +484,17 @@ __global__ void __launch_bounds__(256) tomo_bp_voxel_kernel(float* __restrict__ 
 // Whether the kernels with shared row sums take the call: cells no larger than
 // the pixels (a footprint then spans at most two pixels of any plane between
 // source and panel) and no smaller than 0.6 of them (a voxel at most two cells
-// at magnifications to 1.2).  Elsewhere their threads fall back to whole
-// rectangles, with fewer of them in flight.  Pixels of 0.4 mm, forward and back, one
-// rectangle per thread and shared rows: cells of 0.25 mm 4.55 and 1.58 ms (64 x
-// 256 x 512 voxels, 25 views), 0.24 mm 466 and 227 us (56 x 166 x 200, 10 views);
-// 0.52 mm 221 and 336 us (18 x 127 x 273, 19 views), 0.57 mm 137 and 310 us (26 x
-// 121 x 225, 9 views).
+// at magnifications to 1.2), with a margin for sizes rounded to FP32 (0.24 over
+// 0.4 is 0.59999998).  Elsewhere their threads fall back to whole rectangles,
+// with fewer of them in flight.  Pixels of 0.4 mm, forward and back, one rectangle
+// per thread and shared rows: cells of 0.25 mm 4.55 and 1.63 ms (64 x 256 x 512
+// voxels, 25 views), 0.24 mm 466 and 232 us (56 x 166 x 200, 10 views); 0.52 mm
+// 221 and 336 us (18 x 127 x 273, 19 views), 0.57 mm 137 and 310 us (26 x 121 x 225,
+// 9 views).
 bool shared_rows(const ctp_geometry& g) {
+    const double finest = 0.6 * (1 - 1e-6);
     const double u = fabs((double)g.du / g.dx), v = fabs((double)g.dv / g.dy);
-    return u <= 1.0 && v <= 1.0 && u >= 0.6 && v >= 0.6;
+    return u <= 1.0 && v <= 1.0 && u >= finest && v >= finest;
 }
 
 }  // namespace

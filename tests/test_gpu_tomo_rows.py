@@ -1,6 +1,6 @@
 """Row-sharing tomosynthesis kernels at the sizes where they can go wrong: rows
-and planes around their tiles, and footprints on both sides of the 2 x 2 and
-3 x 3 cells that they hold; against the FP64 oracle."""
+and planes around their tiles, footprints on both sides of the 2 x 2 and 3 x 3
+cells that they hold, borders and weights; against the FP64 oracle."""
 import numpy as np
 import pytest
 
@@ -29,7 +29,8 @@ def dev(a):
                                                  (64, 40, 17, 31, 33, 0.45),
                                                  (50, 37, 8, 40, 24, 1.1)])
 def test_tomo_rows(nx, ny, nz, nu, nv, cell, oracle):
-    """Rows and planes around the kernels' tiles; 0.45 and 1.1 mm cells take one rectangle per thread."""
+    """Rows and planes around the kernels' tiles; 0.45 and 1.1 mm cells take one
+    rectangle per thread."""
     from cases import Proj
 
     from ctprojector_b200 import synthetic as S
@@ -118,3 +119,27 @@ def test_tomo_ray_length_weight_is_rounded_once():
     v = (np.arange(m) - 0.5 - (m - 1) / 2) * 0.5 - s[1]
     ref = (1 / abs(s[2]) * np.sqrt(u * u + v[:, None] ** 2 + s[2] ** 2)).astype(np.float32)
     assert (out != ref).mean() < 1e-3
+
+
+@pytest.mark.parametrize("cell,det_z", [(0.24, -25.0), (0.25, -170.0), (0.4, 1.5)])
+def test_tomo_footprints_past_the_rows(cell, det_z, oracle):
+    """Both sides of the footprints that the rows hold, within the sizes that
+    take them: 0.24 mm is 0.6 of a pixel; 0.25 mm under a panel far below, where
+    voxels span 2.1 cells and more (magnification above 1.3); and a panel inside
+    the volume, past which the footprints of 0.4 mm cells exceed a pixel."""
+    from cases import Proj
+
+    from ctprojector_b200 import synthetic as S
+
+    p = Proj(nx=45, ny=37, nz=21, dx=0.4, dy=0.4, dz=1.0, nu=90, nv=70, du=cell, dv=cell, nview=7)
+    dc, sr = S.tomo_geometry(7, 30.0, 500.0, det_z)
+    rng = np.random.default_rng(9)
+    img = rng.uniform(0, 1, (1, 21, 37, 45)).astype(np.float32)
+    prj = rng.uniform(0, 1, (1, 7, 70, 90)).astype(np.float32)
+    assert rel_l2(tomo_call("distance_driven_fp", p, img, dc, sr), oracle.tomo_fp(p, img, dc, sr)) <= TOL_WIDE
+    assert rel_l2(tomo_call("distance_driven_bp", p, prj, dc, sr), oracle.tomo_bp(p, prj, dc, sr)) <= TOL_WIDE
+
+
+# whole rectangles take their edges in FP32 from the array's corner: up to 90 cells
+# of 2^-24 between a footprint's two edges
+TOL_WIDE = 90 * 2.0**-24
