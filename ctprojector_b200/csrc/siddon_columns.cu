@@ -430,9 +430,10 @@ __host__ __device__ __forceinline__ int sum_rows(int nv) {
 }
 
 // Running sums over the rows of every detector column of the upright views,
-// each cell times its ray's length: P[b][view][run][k][iu] = sum over the run's
-// first k cells, in FP64, stored FP32 (row pitch a multiple of 4 cells); and per
-// column the reciprocal steps of its x-y line.  stats[b][view][run][block]: the
+// each cell times its ray's length: P[b][view][run][k][iu] = sum over the cells
+// from the run's middle to k (negative before it: only differences are used, and
+// these numbers are half as large), in FP64, stored FP32 (row pitch a multiple of
+// 4 cells); and per column the reciprocal steps of its x-y line.  stats[b][view][run][block]: the
 // sum of the cells' magnitudes (each cell once) and the largest sum's, infinite
 // when a cell is not finite; zeros for views that are not upright.
 template <typename Tin>
@@ -460,18 +461,31 @@ __global__ void __launch_bounds__(128) columns_prefix_kernel(float* __restrict__
         const int own = run_i + 1 < runs ? kSumStep : rows;  // rows that the next run does not start in
         const Tin* src = prj + (((size_t)b * nview + view) * d.nv + va) * d.nu + iu;
         float* out = P + (((size_t)b * nviews + vi) * sum_rows(d.nv) + run_i * (kSumRows + 1)) * pitch + iu;
-        out[0] = 0.f;
-        double run = 0.0;
-#pragma unroll 8
-        for (int v = 0; v < rows; ++v) {
+        auto cell = [&](int v) {
             const float z = fmaf((float)(va + v), kv, k0);
             const float p = ldf(src + (size_t)v * d.nu) * sqrtf(fmaf(z, z, l2));
-            run += (double)p;
             if (v < own) mag += fabsf(p);
-            top = fmaxf(top, fabsf((float)run));
-            out[(size_t)(v + 1) * pitch] = (float)run;
+            return (double)p;
+        };
+        auto put = [&](int k, double sum) {
+            const float f = (float)sum;
+            top = fmaxf(top, isfinite(f) ? fabsf(f) : INFINITY);
+            out[(size_t)k * pitch] = f;
+        };
+        const int mid = rows / 2;
+        double run = 0.0;
+        put(mid, 0.0);
+#pragma unroll 8
+        for (int v = mid; v < rows; ++v) {
+            run += cell(v);
+            put(v + 1, run);
         }
-        if (!isfinite((float)run) || isinf(top)) top = INFINITY;
+        run = 0.0;
+#pragma unroll 8
+        for (int v = mid - 1; v >= 0; --v) {
+            run -= cell(v);
+            put(v, run);
+        }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -493,9 +507,9 @@ __global__ void __launch_bounds__(128) columns_prefix_kernel(float* __restrict__
 // sum that is not finite would spread over the column, and one far above the
 // other cells would cost them their bits.  A voxel's sum is a difference of two
 // FP32 numbers of the largest sum's size, so it may be off by 2^-24 of that in
-// one view; kOutlier times the cells of a run at their mean magnitude (over the
-// views at hand) bounds this to 2^-24 x 32 x 96 = 2e-4 of a mean cell a view,
-// 4e-7 of a voxel that 360 views meet with a cell or two each.  Sums reach
+// one view; kOutlier times the cells of half a run at their mean magnitude (over
+// the views at hand) bounds this to 2^-24 x 32 x 48 = 1e-4 of a mean cell a view,
+// 2e-7 of a voxel that 360 views meet with a cell or two each.  Sums reach
 // one over the share of the columns that the object covers: 3% stay.
 // One block; sums in a fixed order.
 constexpr float kOutlier = 32.f;
@@ -526,7 +540,7 @@ __global__ void __launch_bounds__(256) retire_views_kernel(UprightView* __restri
         __syncthreads();
     }
     const float mean = s_mag[0] / ((float)max(s_up[0], 1) * (float)nbatch * (float)d.nu * (float)d.nv);
-    const float most = kOutlier * (float)min(d.nv, kSumRows) * mean;
+    const float most = kOutlier * 0.5f * (float)min(d.nv, kSumRows) * mean;
     for (int vi = threadIdx.x; vi < nviews; vi += blockDim.x) {
         if (!views[view0 + vi].upright) continue;
         bool keep = true;
