@@ -40,9 +40,22 @@ constexpr int kMagicBits = 0x4B400000;
 
 __device__ __forceinline__ int floor_bits(float x) { return __float_as_int(__fadd_rd(x, kMagic)); }
 
+// Whether a detector column's line runs along a grid plane of one axis (within
+// 1e-5 voxels of it from the source, s, to the panel, s + d0 + iu du).  To which
+// side such rays belong is decided ray by ray, where each enters the grid
+// (siddon.cu init_ray: steps below 1e-6 count as none), as for the middle column
+// of an odd detector over an even grid at 0, 90, 180 and 270 degrees.
+__device__ __forceinline__ bool along_plane(double s, double d0, double du, int nu) {
+    const double at = rint(-d0 / du);
+    if (!(at >= 0.0 && at < nu)) return false;
+    const double d = fabs(d0 + at * du);
+    return d < 1e-5 && fabs(s - rint(s)) < 1e-5 + d;
+}
+
 // One block.  Upright: v along z, u across z, and every corner of the grid at
 // alpha in (1e-3, 1]: the source outside the grid with the grid in front of
-// it and before the panel, so that no ray ends inside the grid.
+// it and before the panel, so that no ray ends inside the grid; and no line
+// along a grid plane.
 __global__ void __launch_bounds__(256) view_setup_kernel(UprightView* __restrict__ out, int* __restrict__ rest,
                                                          const float* __restrict__ dc, const float* __restrict__ du_,
                                                          const float* __restrict__ dv_, const float* __restrict__ sr,
@@ -74,6 +87,7 @@ __global__ void __launch_bounds__(256) view_setup_kernel(UprightView* __restrict
                 const double alpha = (w.ux * py[b] - w.uy * px[a]) / w.det;
                 up = up && alpha > 1e-3 && alpha <= 1.0;
             }
+        up = up && !along_plane(w.sx, w.dx0, w.ux, d.nu) && !along_plane(w.sy, w.dy0, w.uy, d.nu);
         w.upright = up ? 1 : 0;
         out[view] = w;
         if (!up) rest[1 + atomicAdd(&n_rest, 1)] = view;

@@ -174,3 +174,13 @@ def test_no_less_exact_than_ray_by_ray(oracle, monkeypatch):
             m.setattr(_device, "_io_flags", lambda a, b: flags(a, b) & ~SIDDON_COLUMNS)
             rays = rel_l2(cone.siddon_bp_arbitrary(p, x, *dev).cpu().numpy(), ref)
         assert columns <= 1.02 * rays, (nview, columns, rays)  # (both are sums of some 1e6 roundings)
+
+
+@pytest.mark.parametrize("nx,nu,nv", [(150, 195, 31), (64, 65, 33), (32, 33, 64)])
+def test_rays_along_grid_planes(nx, nu, nv, oracle):
+    """An odd detector over an even grid, views at 0, 90, 180 and 270 degrees: the
+    middle column's rays run along the plane between two pixel columns, and belong
+    to the side on which each enters the grid."""
+    p = scan(nx, nx, 32, nu, nv, nview=12, pixel=358.0 / nx, dz=1.1)
+    check(p, helix(p, feed=35.0), oracle)
+    check(p, helix(p), oracle)
