@@ -376,7 +376,9 @@ __global__ void __launch_bounds__(256, 5) columns_fp_kernel(Tout* __restrict__ p
             const int pin = ln.dm > 0 ? slab : slab + 1, pout = ln.dm > 0 ? slab + 1 : slab;
             const double aa = (pin - ln.sm) * ln.im, ab = (pout - ln.sm) * ln.im;
             const double ya = ln.so + aa * ln.dO, yb = ln.so + ab * ln.dO;
-            const int ja = (int)floor(fmin(fmax(ya, -2.0), no + 1.0)), jb = (int)floor(fmin(fmax(yb, -2.0), no + 1.0));
+            int ja = (int)floor(fmin(fmax(ya, -2.0), no + 1.0)), jb = (int)floor(fmin(fmax(yb, -2.0), no + 1.0));
+            // from corner to corner (45 degrees) rounding may show the cells on both sides of the one crossed
+            if (abs(jb - ja) > 1) ja = jb = (ja + jb) / 2;
             double ac = ab;
             if (ja != jb) ac = fmin(fmax((max(ja, jb) - ln.so) * ln.io, aa), ab);
             const bool f1 = in && ja >= 0 && ja < no, f2 = in && ja != jb && jb >= 0 && jb < no;

@@ -184,3 +184,11 @@ def test_rays_along_grid_planes(nx, nu, nv, oracle):
     p = scan(nx, nx, 32, nu, nv, nview=12, pixel=358.0 / nx, dz=1.1)
     check(p, helix(p, feed=35.0), oracle)
     check(p, helix(p), oracle)
+
+
+@pytest.mark.parametrize("n,nu", [(64, 65), (32, 33), (150, 195), (33, 47)])
+def test_rays_through_pixel_corners(n, nu, oracle):
+    """The middle column at 45 degrees runs from corner to corner of square pixels."""
+    p = scan(n, n, 32, nu, 32, nview=8, pixel=358.0 / n, dz=1.1)
+    check(p, helix(p, feed=35.0), oracle)
+    check(p, helix(p), oracle)
