@@ -52,10 +52,22 @@ __device__ __forceinline__ bool along_plane(double s, double d0, double du, int 
     return d < 1e-5 && fabs(s - rint(s)) < 1e-5 + d;
 }
 
+// The same for a detector row at the source's height, z by z: the kernels below
+// take z in FP32, and a ray that hardly rises near a plane would lie on the side
+// that the rounding says.  (Exactly level on exactly a plane, as in the middle row
+// of a circular scan, all agree.)
+__device__ __forceinline__ bool level_at_plane(double zs, double k0, double kv, int nv, int nz) {
+    const double at = rint(-k0 / kv);
+    if (!(at >= 0.0 && at < nv)) return false;
+    const double d = fabs(k0 + at * kv), off = fabs(zs - rint(zs));
+    const double rounding = 2.4e-7 * (nz + 1.0);  // 2^-22 of the largest z
+    return d < 1e-3 && off < rounding + d && !(off == 0.0 && d < 1e-12);
+}
+
 // One block.  Upright: v along z, u across z, and every corner of the grid at
 // alpha in (1e-3, 1]: the source outside the grid with the grid in front of
-// it and before the panel, so that no ray ends inside the grid; and no line
-// along a grid plane.
+// it and before the panel, so that no ray ends inside the grid; and no line or
+// row along a grid plane.
 __global__ void __launch_bounds__(256) view_setup_kernel(UprightView* __restrict__ out, int* __restrict__ rest,
                                                          const float* __restrict__ dc, const float* __restrict__ du_,
                                                          const float* __restrict__ dv_, const float* __restrict__ sr,
@@ -87,7 +99,8 @@ __global__ void __launch_bounds__(256) view_setup_kernel(UprightView* __restrict
                 const double alpha = (w.ux * py[b] - w.uy * px[a]) / w.det;
                 up = up && alpha > 1e-3 && alpha <= 1.0;
             }
-        up = up && !along_plane(w.sx, w.dx0, w.ux, d.nu) && !along_plane(w.sy, w.dy0, w.uy, d.nu);
+        up = up && !along_plane(w.sx, w.dx0, w.ux, d.nu) && !along_plane(w.sy, w.dy0, w.uy, d.nu) &&
+             !level_at_plane(w.zs, w.k0, w.kv, d.nv, g.nz);
         w.upright = up ? 1 : 0;
         out[view] = w;
         if (!up) rest[1 + atomicAdd(&n_rest, 1)] = view;
