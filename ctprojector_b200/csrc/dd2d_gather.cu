@@ -664,7 +664,9 @@ __global__ void __launch_bounds__(256, (S == 4 ? 3 : 4)) gather_bp_kernel(const 
                             typename L::Point t = L::zero_point();
                             if (!(a <= 0.f)) L::scale_add(t, prev, a);
                             if (!(b <= 0.f)) L::scale_add(t, v, b);
-                            for (int i = 1; i < n; ++i) L::scale_add(t, L::value(at_prev + i * step, plane), 1.f);
+                            if (n > 1) L::scale_add(t, L::value(at_prev + step, plane), 1.f);
+                            if (n > 2)
+                                for (int i = 2; i < n; ++i) L::scale_add(t, L::value(at_prev + i * step, plane), 1.f);
                             acc.add(k - 1, t);
                         }
                         prev = v;
