@@ -55,13 +55,15 @@ __device__ __forceinline__ bool along_plane(double s, double d0, double du, int 
 // The same for a detector row at the source's height, z by z: the kernels below
 // take z in FP32, and a ray that hardly rises near a plane would lie on the side
 // that the rounding says.  (Exactly level on exactly a plane, as in the middle row
-// of a circular scan, all agree.)
+// of a circular scan, all agree; the lowest plane is at 0, where FP32 tells every
+// side.)
 __device__ __forceinline__ bool level_at_plane(double zs, double k0, double kv, int nv, int nz) {
     const double at = rint(-k0 / kv);
     if (!(at >= 0.0 && at < nv)) return false;
-    const double d = fabs(k0 + at * kv), off = fabs(zs - rint(zs));
-    const double rounding = 2.4e-7 * (nz + 1.0);  // 2^-22 of the largest z
-    return d < 1e-3 && off < rounding + d && !(off == 0.0 && d < 1e-12);
+    const double plane = rint(zs), d = fabs(k0 + at * kv), off = fabs(zs - plane);
+    if (!(plane >= 0.0 && plane <= nz) || (off == 0.0 && d < 1e-12)) return false;
+    const double rounding = plane > 0.0 ? 2.4e-7 * (nz + 1.0) : 0.0;  // 2^-22 of the largest z
+    return d < 1e-3 && off < rounding + d;
 }
 
 // One block.  Upright: v along z, u across z, and every corner of the grid at
@@ -634,10 +636,11 @@ __device__ __forceinline__ float lds_f32(unsigned addr) {
     return v;
 }
 
-// a * b + c clamped to [0, 1] (NaN to 0), and a * b + c rounded up.
+// a * b + c rounded up and clamped to [0, 1] (NaN to 0): above an integer stays
+// above it, for the ceiling that follows.
 __device__ __forceinline__ float fma_sat(float a, float b, float c) {
     float y;
-    asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+    asm("fma.rp.sat.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
     return y;
 }
 

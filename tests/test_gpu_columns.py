@@ -194,10 +194,10 @@ def test_rays_through_pixel_corners(n, nu, oracle):
     check(p, helix(p), oracle)
 
 
-@pytest.mark.parametrize("cz", [-1.665, -1.664, -1.66, 0.555, 0.5551])
+@pytest.mark.parametrize("cz", [-1.665, -1.664, -1.66, 0.555, 0.5551, 4.995, 4.9949999, 4.9950005, -4.995, -4.9950005])
 def test_level_rays_beside_slice_planes(cz, oracle):
     """The middle row of an odd panel is level at the source's height, here at
-    1.665 / 1.11 = 1.5 slices and nearly so from the middle of nine: 7e-8, 9e-4 and
-    more of a slice from a plane."""
+    1.665 / 1.11 = 1.5 slices and nearly so from the middle of nine (7e-8, 9e-4 and
+    more of a slice from a plane), and at the lowest and the highest plane."""
     p = scan(40, 40, 9, 52, 33, nview=10, pixel=9.0, dz=1.11, cz=cz)
     check(p, helix(p), oracle)
