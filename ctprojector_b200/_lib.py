@@ -33,6 +33,7 @@ FLAG_OUT_BF16 = 0x40
 FLAG_OUT_FP16 = 0x80
 FLAG_FILTER_EXACT = 0x100
 FLAG_SUBTRACT = 0x400
+FLAG_SIDDON_COLUMNS = 0x800
 FLAG_TOMO_FIRST_VIEW_KERNEL = 0x200
 
 TYPE_FBP = 0x1

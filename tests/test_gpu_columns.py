@@ -201,3 +201,35 @@ def test_level_rays_beside_slice_planes(cz, oracle):
     more of a slice from a plane), and at the lowest and the highest plane."""
     p = scan(40, 40, 9, 52, 33, nview=10, pixel=9.0, dz=1.11, cz=cz)
     check(p, helix(p), oracle)
+
+
+def test_columns_by_their_own_size_rule(oracle, monkeypatch):
+    """A scan that both size rules accept by themselves: the forward projection's
+    bits are those of the flagged call, not those of the rays (views that a
+    rounding of the detector axis keeps from being upright)."""
+    from ctprojector_b200.projector import _device
+    from ctprojector_b200.projector.cupy import cone
+
+    p = scan(128, 128, 32, 64, 48, nview=300, pixel=2.8, dz=1.2, cell=14.0, row=1.6)
+    geo = helix(p, feed=20.0)
+    rng = np.random.default_rng(0)
+    img = rng.uniform(0, 1, (1, p.nz, p.ny, p.nx)).astype(np.float32)
+    prj = rng.uniform(0, 1, (1, p.nview, p.nv, p.nu)).astype(np.float32)
+    flags = _device._io_flags
+
+    def run(geo):
+        dev = [torch.tensor(a, device="cuda") for a in geo]
+        return (cone.siddon_fp_arbitrary(p, torch.tensor(img, device="cuda"), *dev).cpu().numpy(),
+                cone.siddon_bp_arbitrary(p, torch.tensor(prj, device="cuda"), *dev).cpu().numpy())
+
+    flagged = run(geo)
+    with monkeypatch.context() as m:
+        m.setattr(_device, "_io_flags", lambda a, b: flags(a, b) & ~SIDDON_COLUMNS)
+        fp, bp = run(geo)
+        tilted = [a.copy() for a in geo]
+        tilted[1][:, 2] = 1e-12
+        rays, _ = run(tilted)
+    np.testing.assert_array_equal(fp, flagged[0])
+    assert not np.array_equal(fp, rays)
+    assert rel_l2(fp, oracle.siddon_fp(p, img, *geo)) <= TOL
+    assert rel_l2(bp, oracle.siddon_bp(p, prj, *geo)) <= TOL

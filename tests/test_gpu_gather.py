@@ -76,7 +76,8 @@ def test_more_views_than_one_list(geom, oracle):
 
 @pytest.mark.parametrize("pixel", [0.1, 6.0])
 def test_fan_small_and_wide_tiles(pixel, oracle):
-    """6 mm pixels: a tile spans more than the series of atan is used for."""
+    """6 mm pixels: a tile spans more than the series of atan is used for (its
+    12 mm cells are past those that the adjoint takes: see the widest ones)."""
     p = proj("fan", 40, 40, 70, pixel=pixel)
     check(p, angles(36, "fan"), "fan", oracle, 2)
 
