@@ -69,11 +69,12 @@ __device__ __forceinline__ bool level_at_plane(double zs, double k0, double kv, 
 // One block.  Upright: v along z, u across z, and every corner of the grid at
 // alpha in (1e-3, 1]: the source outside the grid with the grid in front of
 // it and before the panel, so that no ray ends inside the grid; and no line or
-// row along a grid plane.
+// row along a grid plane.  rows_up: rows that go down are counted from the other
+// end of the panel.
 __global__ void __launch_bounds__(256) view_setup_kernel(UprightView* __restrict__ out, int* __restrict__ rest,
                                                          const float* __restrict__ dc, const float* __restrict__ du_,
                                                          const float* __restrict__ dv_, const float* __restrict__ sr,
-                                                         int nview, Grid g, Det d) {
+                                                         int nview, Grid g, Det d, int rows_up) {
     __shared__ int n_rest;
     if (threadIdx.x == 0) n_rest = 0;
     __syncthreads();
@@ -104,6 +105,11 @@ __global__ void __launch_bounds__(256) view_setup_kernel(UprightView* __restrict
         up = up && !along_plane(w.sx, w.dx0, w.ux, d.nu) && !along_plane(w.sy, w.dy0, w.uy, d.nu) &&
              !level_at_plane(w.zs, w.k0, w.kv, d.nv, g.nz);
         w.upright = up ? 1 : 0;
+        w.turned = rows_up && w.kv < 0 ? 1 : 0;
+        if (w.turned) {
+            w.k0 += (d.nv - 1) * w.kv;
+            w.kv = -w.kv;
+        }
         out[view] = w;
         if (!up) rest[1 + atomicAdd(&n_rest, 1)] = view;
     }
@@ -490,11 +496,12 @@ __global__ void __launch_bounds__(128) columns_prefix_kernel(float* __restrict__
         const float k0 = (float)(w.k0 * g.dz), kv = (float)(w.kv * g.dz);
         const int va = run_i * kSumStep, rows = min(kSumRows, d.nv - va);
         const int own = run_i + 1 < runs ? kSumStep : rows;  // rows that the next run does not start in
-        const Tin* src = prj + (((size_t)b * nview + view) * d.nv + va) * d.nu + iu;
+        const Tin* src = prj + (((size_t)b * nview + view) * d.nv) * d.nu + iu;
         float* out = P + (((size_t)b * nviews + vi) * sum_rows(d.nv) + run_i * (kSumRows + 1)) * pitch + iu;
         auto cell = [&](int v) {
             const float z = fmaf((float)(va + v), kv, k0);
-            const float p = ldf(src + (size_t)v * d.nu) * sqrtf(fmaf(z, z, l2));
+            const int row = w.turned ? d.nv - 1 - (va + v) : va + v;
+            const float p = ldf(src + (size_t)row * d.nu) * sqrtf(fmaf(z, z, l2));
             if (v < own) mag += fabsf(p);
             return (double)p;
         };
@@ -607,7 +614,7 @@ struct BpView {
     float ar;                       // alpha of the tile's centre (alphas are kept relative to it)
     float zz0;                      // the z range's first plane minus the source's z
     float vc;                       // row coordinate of the source's z plane, from the staged rows' base
-    float ikv, sgn;                 // 1 / kv and its sign
+    float ikv;                      // 1 / kv
     float kbf, kvf;                 // kb and kv in FP32
     double bx, by;                  // tile origin minus the source, x and y
     double zd, kb, kv;              // zz0 in FP64; z rise over alpha 0 .. 1 of the staged rows: kb + k kv
@@ -683,7 +690,6 @@ __device__ __forceinline__ bool bp_view(const UprightView& w, int tx0, int ty0, 
     V.by = oy;
     V.zz0 = (float)(z0 - w.zs);
     V.ikv = (float)(1.0 / w.kv);
-    V.sgn = w.kv > 0 ? 1.f : -1.f;
     // z reached by the rows 0 and nv - 1 over the tile's alphas
     const double ka = w.k0, kb = w.k0 + (d.nv - 1) * w.kv;
     const double klo = fmin(ka, kb), khi = fmax(ka, kb);
@@ -740,7 +746,7 @@ __global__ void __launch_bounds__(128) bp_fit_kernel(UprightView* __restrict__ v
 // views' arithmetic).  Per detector column whose line crosses the pixel,
 // between alphas aA and aB:
 //   the rays of the column below the plane z at alpha a are the rows below
-//   v(z, a) = (z - zs) / (a kv) - k0 / kv (kv > 0), so the sum of the rays below z is
+//   v(z, a) = (z - zs) / (a kv) - k0 / kv (kv > 0: view_setup_kernel), so the sum of the rays below z is
 //   the running sum at ceil(v), the same at both ends unless a row passes
 //   through the plane inside the pixel; such rows count with the part of the
 //   segment below (noted in a bit mask, added after the planes' loop).  The
@@ -868,7 +874,6 @@ __global__ void __launch_bounds__(256, 2) columns_bp_kernel(float* __restrict__ 
         const float chord = fminf(fminf(wx, wy), fminf(wx + e, wy - e));
         if (!(chord > 0.f)) return;
         const float lo = e < 0.f ? fmaf(ky, L.dy, L.y0) + fminf(L.dy, 0.f) : fmaf(kx, L.dx, L.x0) + fminf(L.dx, 0.f);
-        const float da = chord * V.sgn;
         const float aA = V.ar + lo, aB = V.ar + (lo + chord);
         const float gA = __fdividef(V.ikv, aA), gB = __fdividef(V.ikv, aB);
         const int g0 = V.g0, g1 = V.g1;
@@ -897,7 +902,7 @@ __global__ void __launch_bounds__(256, 2) columns_bp_kernel(float* __restrict__ 
             for (int q = 1; q <= kBpGroup; ++q) s[q] = plane(grp * kBpGroup + q);
 #pragma unroll
             for (int q = 0; q < kBpGroup; ++q)
-                acc[grp * kBpGroup + q] = fmaf(s[q + 1] - s[q], da, acc[grp * kBpGroup + q]);
+                acc[grp * kBpGroup + q] = fmaf(s[q + 1] - s[q], chord, acc[grp * kBpGroup + q]);
             below = s[kBpGroup];
         }
         // rows through a plane: the part of their segment below it, relative to
@@ -921,7 +926,7 @@ __global__ void __launch_bounds__(256, 2) columns_bp_kernel(float* __restrict__ 
                                                        chord * kappa));
                 part = fmaf(col[(k + 1) * kBpWin] - col[k * kBpWin], kA > kB ? f - 1.f : 1.f - f, part);
             }
-            s_split[q * 256 + tid] += part * da;
+            s_split[q * 256 + tid] += part * chord;
         }
     };
 
@@ -1043,11 +1048,11 @@ int launch_columns_fp(void* prj, const void* img, const ctp_geometry& g, unsigne
 }
 
 int setup_views(ColumnsPlan& plan, char* base, const float* dc, const float* du_, const float* dv_, const float* sr,
-                const ctp_geometry& g, cudaStream_t s) {
+                const ctp_geometry& g, bool rows_up, cudaStream_t s) {
     plan.views = reinterpret_cast<UprightView*>(base);
     plan.rest = reinterpret_cast<int*>(base + align_up(g.nview * sizeof(UprightView)));
     view_setup_kernel<<<1, 256, 0, s>>>(plan.views, plan.rest, dc, du_, dv_, sr, (int)g.nview, make_grid(g),
-                                        make_det(g));
+                                        make_det(g), rows_up ? 1 : 0);
     return check_launch("view_setup_kernel");
 }
 
@@ -1076,7 +1081,7 @@ size_t columns_fp_bytes(const ctp_geometry& g, unsigned flags) {
 
 int columns_fp(ColumnsPlan& plan, char* scratch, void* prj, const void* img, const float* dc, const float* du_,
                const float* dv_, const float* sr, const ctp_geometry& g, unsigned flags, cudaStream_t s) {
-    int rc = setup_views(plan, scratch, dc, du_, dv_, sr, g, s);
+    int rc = setup_views(plan, scratch, dc, du_, dv_, sr, g, false, s);
     if (rc) return rc;
     char* copy = scratch + setup_bytes(g);
     if (flags & CTP_FLAG_IN_BF16)
@@ -1130,7 +1135,7 @@ size_t columns_bp_bytes(const ctp_geometry& g) {
 
 int columns_bp(ColumnsPlan& plan, char* scratch, float* img, const void* prj, const float* dc, const float* du_,
                const float* dv_, const float* sr, const ctp_geometry& g, unsigned flags, cudaStream_t s) {
-    int rc = setup_views(plan, scratch, dc, du_, dv_, sr, g, s);
+    int rc = setup_views(plan, scratch, dc, du_, dv_, sr, g, true, s);
     if (rc) return rc;
     const size_t nv = bp_views(g);
     char* p = scratch + setup_bytes(g);

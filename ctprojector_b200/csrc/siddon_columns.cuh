@@ -15,6 +15,7 @@ struct UprightView {
     double k0, kv;
     double det;   // (ux, uy) x (dx0, dy0)
     int upright;  // 0: the ray-driven kernels take this view
+    int turned;   // k0 and kv count the rows from the panel's other end (columns_bp)
 };
 
 // Device memory of one call: the views, and rest[0] = the number of views that

@@ -233,3 +233,18 @@ def test_columns_by_their_own_size_rule(oracle, monkeypatch):
     assert not np.array_equal(fp, rays)
     assert rel_l2(fp, oracle.siddon_fp(p, img, *geo)) <= TOL
     assert rel_l2(bp, oracle.siddon_bp(p, prj, *geo)) <= TOL
+
+
+@pytest.mark.parametrize("nv", [2, 25, 57])
+@pytest.mark.parametrize("flip", ["axis", "pitch"])
+def test_level_rows_of_a_panel_upside_down(flip, nv, oracle):
+    """Rows on slice planes exactly, with rows that go down: they belong to the
+    slice above, as they do with rows that go up."""
+    p = scan(33, 40, 32, 50, nv, dz=1.0, off_v=0.5 if nv == 2 else 0.0)
+    geo = helix(p, feed=16.0)
+    if flip == "axis":
+        geo[2] = -geo[2]
+    else:
+        p.dv = -p.dv
+    check(p, geo, oracle)
+    check(p, [*helix(p)[:2], geo[2], helix(p)[3]], oracle)
