@@ -153,7 +153,7 @@ FILTER_NOTE = ("hann ramp filter in exact mode (FP64 arithmetic, one launch; ~1e
 
 # the launches behind each timed projector operation (the roofline names the dominant one)
 ROOFLINE_KERNEL = {
-    "fp": "dd2d_fp_stream_kernel (with its edge-table, view-order, transpose and line-table launches)",
+    "fp": "dd2d_fp_stream_kernel (with its edge-table, transpose and line-table launches)",
     "bp": "gather_bp_kernel",
     "bp_fbp": "gather_bp_kernel (FBP weighting)",
 }

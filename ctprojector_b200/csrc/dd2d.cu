@@ -15,9 +15,10 @@
 //  * dd_table_kernel evaluates, once per call and in FP64, the footprint edges
 //    of every detector-cell edge ray of every view as lines x(row) = A + B*t in
 //    image coordinates (t = row - anchor) and the ray-length factor L per
-//    cell.  The forward projector
-//    and its exact transpose read the same FP32 table entries, so both see
-//    bit-identical footprints.
+//    cell.  The forward projectors and the general transpose here read the
+//    same FP32 table entries; the tiled transpose (dd2d_gather.cu) takes the
+//    footprints from FP64 constants of its tiles and agrees with them to the
+//    rounding of both (the adjoint identity within 1e-6).
 //  * Forward projection streams the image's line tables through shared memory
 //    (dd2d_fp_stream_kernel).  Views traced along x read a transposed copy of
 //    the image so that those walks are row reads too.

@@ -37,14 +37,15 @@
 // the y-edge ones (a part of 32 views has some of each: 2 x 168 x 140, 255 views,
 // filtered back projection 56 -> 52 us).  No atomics; every sum in a fixed order.
 //
-// Measured (B200): parallel mean, 16 x 512^2, 720 views 1.72 -> 1.48 ms against
+// Measured (B200): parallel mean, 16 x 512^2, 720 views 1.72 -> 1.42 ms against
 // two sets of accumulators and one 8-byte read per slice and lookup (bound now
-// by shared-memory wavefronts, 74%, at 61% issue); fan mean, 4 x 512^2, 984 views
-// 1.39 -> 1.15 ms, with the edges' angles relative to the tile's centre by a
-// short series instead of an atanf each (53% issue: latency at 3 CTAs per SM);
-// adjoint, fan 2 x 512^2, 984 views 12.6 -> 0.95 ms and parallel 3 x 317 x 413,
-// 501 views 3.4 -> 0.2 ms against the kernel that intersects every cell with
-// every pixel; pixel-driven fan, 4 x 512^2, 984 views 3.6 -> 0.85 ms.
+// by shared-memory wavefronts, 76%, at 68% issue); fan mean, 4 x 512^2, 984 views
+// 1.39 -> 0.94 ms, with the edges' angles relative to the tile's centre by a
+// short series instead of an atanf each (57% issue: the window's tables leave two
+// CTAs per SM, where the registers allow three); adjoint, fan 2 x 512^2, 984 views
+// 12.6 -> 0.97 ms and parallel 3 x 317 x 413, 501 views 3.4 -> 0.21 ms against the
+// kernel that intersects every cell with every pixel (as differences of F: 0.85
+// and 0.17 ms); pixel-driven fan, 4 x 512^2, 984 views 3.6 -> 0.80 ms.
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -848,7 +849,8 @@ int gather_window(const ctp_geometry& g, int geom, double* zmax) {
     return win <= kMaxWin ? win : 0;
 }
 
-// CTAs resident on an SM (the kernels' registers).
+// CTAs resident on an SM by the kernels' registers; windows of more than 103 cells
+// (fan, S = 4) leave one less by shared memory.
 int ctas_per_sm(int S) { return S == 4 ? 3 : 4; }
 
 int sm_count() {
@@ -912,7 +914,8 @@ int gather_parts(const ctp_geometry& g, int geom, int& vper) {
     return (int)((g.nview + vper - 1) / vper);
 }
 
-// Fan mean: the cells' weights, in the room of a weighted copy of the sinogram.
+// Fan mean: the cells' weights of a view, in the room that the workspace query
+// keeps for a weighted copy of the sinogram (the general kernel's).
 size_t weight_bytes(const ctp_geometry& g, int geom, GatherMode mode) {
     if (geom != 0 || mode == kGatherFbp || mode == kGatherPixel) return 0;
     if (mode == kGatherAdjoint) return align_up(2 * g.nview * g.nu * sizeof(float));

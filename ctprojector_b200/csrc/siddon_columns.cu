@@ -763,11 +763,11 @@ __global__ void __launch_bounds__(128) bp_fit_kernel(UprightView* __restrict__ v
 //
 // Bound by issue: per plane and crossing line two saturating multiply-adds, two
 // directed roundings, a compare and a read.  The same volume and views: 14.9 ms
-// ray by ray (siddon_bp_kernel's atomics), 6.45 ms here; 33 x 187 x 201 voxels,
-// 97 views of 251 x 37 cells: 362 -> 350 us with the set-up launches.  Measured
-// and not taken, same volume: columns as the rows of the staged window (bank
-// conflicts) 6.74 ms; one view between barriers 6.10; three blocks per SM at 80
-// registers 6.56; two threads per pixel, every other line each, 9.2.
+// ray by ray (siddon_bp_kernel's atomics), 6.40 ms here.  Measured and not taken,
+// same volume, when the kernel took 5.96 ms (chords of FP32 alphas, one sum over
+// the views): columns as the rows of the staged window (bank conflicts) 6.74 ms;
+// one view between barriers 6.10; three blocks per SM at 80 registers 6.56; two
+// threads per pixel, every other line each, 9.2.
 template <bool ATOMIC>
 __global__ void __launch_bounds__(256, 2) columns_bp_kernel(float* __restrict__ img, const float* __restrict__ P,
                                                             const double2* __restrict__ inv,
