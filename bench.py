@@ -138,10 +138,10 @@ def algorithmic_bytes(nnz_slice: int, nb: int, scan) -> dict:
     return {"fp": proj, "bp": proj, "filter": 4 * 2 * n_prj, "bp_fbp": proj}
 
 
-# ours: launches of our own kernels per step (FP: edge table, view order,
-# transpose, row and column line tables, streamed sweep; BP: gather; filter:
-# one FFT row convolution over every row; FBP BP: gather)
-OUR_LAUNCHES_PER_STEP = 6 + 1 + 1 + 1
+# ours: launches of our own kernels per step (FP: edge table with the view
+# order, transpose, row and column line tables, streamed sweep; BP: gather;
+# filter: one FFT row convolution over every row; FBP BP: gather)
+OUR_LAUNCHES_PER_STEP = 5 + 1 + 1 + 1
 
 # The filter of the step runs in exact mode: FP64 arithmetic in one launch
 # (conv_rows_kernel).  The default mode replays the reference's FP32
